@@ -5,12 +5,11 @@
 //
 //   * k_upwind, one thread per (phase, connection): upstream bulk and mean
 //     density;
-//   * k_conn_block, a group of connections per block: thread (row,
-//     connection) builds that row of dF/dXp and dF/dXs of both ends in
-//     shared memory, then thread (column, connection) forms that column of
-//     dt (dF/dXp + dF/dXs dSec_dPri) (DaABpbC, src/DenseMat.cpp:75-94) for
-//     both ends, so that each dSec_dPri entry is read once per connection
-//     end; stored as the connection's off-diagonal blocks;
+//   * k_conn_block, one lane per connection, one warp per end and group of
+//     rows: forms each entry of those rows of dF/dXp and dF/dXs and at once
+//     multiplies it into the rows of dt (dF/dXp + dF/dXs dSec_dPri)
+//     (DaABpbC, src/DenseMat.cpp:75-94), held in registers; stored as the
+//     connection's off-diagonal blocks;
 //   * k_diag_rows, one thread per (row, bulk): the accumulation block plus
 //     every incident connection's diagonal contribution, gathered through a
 //     per-bulk list in connection order, which is the order the reference's
@@ -78,300 +77,387 @@ __global__ void __launch_bounds__(256) k_upwind(const ConnDev C, const ocpf_jac_
     }
 }
 
-// The compact dSec_dPri layout of one bulk: sderivative flags and composition
-// counts of its phases.
-struct SecShape {
-    bool sd[J_NP];
-    int  vn[J_NP];
-    int  ncol;  // rows of its dSec_dPri = columns of its dF/dXs
+// Work split of k_conn_block: a tile of 32 consecutive connections (one per
+// lane) is served by 2 G warps, warp (end, g) forming NR of the NCOM rows of
+// that end's block, all NCOL columns of them in registers; every dF/dXs entry
+// is multiplied into them as it is formed, so that neither the dF/dXs rows
+// nor the product's columns are stored in between. Lanes of a warp hold
+// consecutive connections, whose end bulks are consecutive along a grid line:
+// the dSec_dPri entries come as coalesced 256-byte lines. For 3 and 6
+// components a tile's entries (both ends) are copied asynchronously into
+// shared memory first, 61 KB for 6 components, three tiles an SM in flight.
+//
+// Bound by latency and the issue of ~4,000 unfused FP64 operations of a
+// two-phase connection (FP64 pipe 37 % busy at 12 warps an SM), with ~1 KB of
+// stores and 2 KB of loads beside them. 60 x 220 x 85 bulks, 6 components,
+// whole call: 11.1 ms with the rows and columns through shared memory (one
+// thread per row, then per column), 9.8 ms with this split reading dSec_dPri
+// directly, 7.2 ms staged, 6.2 ms with the next composition's partials
+// prefetched and the quotients batched (div_by). 100,000 bulks: 3 components
+// at 561,000 bulks 3.47 -> 1.28 ms, 9 components 2.42 -> 1.46 ms, 12
+// components 6.76 -> 3.55 ms. Rows a thread: 4 for 3, 6 and 12 components, 5
+// for 9, where 3 or 4 rows took 2.43 ms.
+template <int NCOM>
+struct ConnTile {
+    static constexpr int NCOL  = NCOM + 1;
+    static constexpr int NSEC  = 3 + 2 * (NCOM - 1);     // dSec_dPri rows of a two-phase bulk
+    static constexpr int G     = NCOM <= 4 ? 1 : (NCOM <= 10 ? 2 : 4);  // row groups
+    static constexpr int NR    = (NCOM + G - 1) / G;     // rows of a group; the last group may repeat some
+    static constexpr int TILES = G == 1 ? 2 : 1;         // tiles per block
+    static constexpr int TPT   = 64 * G;                 // threads per tile
+    static constexpr int THREADS = TPT * TILES;
+    static constexpr int MINB    = NCOM <= 7 ? 3 : (NCOM <= 10 ? 2 : 1);
+    // dSec_dPri entries of both ends staged in shared memory
+    static constexpr bool   STAGED  = NCOM <= 7;
+    static constexpr int    NENT    = NSEC * NCOL;
+    static constexpr size_t SEC     = STAGED ? (size_t)2 * NENT * 32 : 0;  // doubles per tile
+    static constexpr size_t XIJ     = (size_t)J_NP * NCOM * 32;
 };
 
-__device__ __forceinline__ SecShape sec_shape(const ocpf_jac_bulk& B, int64_t nb, int64_t n)
+// Per connection and phase, formed once per tile (stage_phase).
+enum : int { Q_DP = 0, Q_XI, Q_MU, Q_Y, Q_MUP, Q_XIP, Q_RHOP, Q_RHOPB, Q_RHOPE, Q_TR, Q_COUNT };
+// flag bits of a connection and phase; bits 8-15 and 16-23 hold the
+// composition counts of the begin and end bulk
+enum : uint32_t { F_EXU = 1, F_UPB = 2, F_EXB = 4, F_EXE = 8, F_SDB = 16, F_SDE = 32, F_BAD = 64, F_SAFE = 128 };
+
+template <int NCOM>
+struct ConnStage {
+    double   sec[ConnTile<NCOM>::SEC + 1];
+    double   x[J_NP * NCOM][32];  // xij of the upstream bulk
+    double   q[J_NP][Q_COUNT][32];
+    uint32_t f[J_NP][32];
+};
+
+// One 8-byte asynchronous copy into shared memory.
+__device__ __forceinline__ void copy8(double* dst, const double* src)
 {
-    SecShape s;
-    s.ncol = 0;
-#pragma unroll
-    for (int j = 0; j < J_NP; j++) {
-        s.sd[j] = B.pSderExist[j * nb + n] != 0;
-        s.vn[j] = (int)B.pVnumCom[j * nb + n];
-        s.ncol += s.vn[j] + (s.sd[j] ? 1 : 0);
-    }
-    return s;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
 }
 
-// Connections per block of k_conn_block and its shared-memory size: the
-// dF/dXs rows of both ends of every connection of the block.
-template <int NCOM>
-struct ConnBlock {
-    static constexpr int NCOL = NCOM + 1;
-    static constexpr int NSEC = 3 + 2 * (NCOM - 1);  // dSec_dPri rows of a two-phase bulk
-    static constexpr int CPB  = NCOM <= 7 ? 16 : (NCOM <= 10 ? 8 : 4);
-    static constexpr int TPC  = NCOL <= 8 ? 8 : 16;  // threads per connection (>= NCOL)
-    static constexpr int THREADS = CPB * TPC;
-    // per connection, staged once: 11 scalars of each phase's upstream
-    // (dP, xi, kr, mu, muP, xiP, rhoP of upstream, begin and end, transJ,
-    // upstream exists), the 9 saturation derivatives of each phase (dPc of
-    // both ends, dKr of upstream), and 5 composition partials of each phase
-    // and component (rhox, xix, mux of upstream, rhox of begin and end)
-    static constexpr int STG = 3 * 11 + 3 * 9 + 3 * 5 * NCOM;
-    static constexpr size_t SMEM =
-        sizeof(double) * (size_t)CPB * (2 * (NSEC * NCOM + NCOM) + STG) + sizeof(int) * CPB * 3;
-    static_assert(NCOL <= TPC, "one thread per column");
-};
-
-// Phase 1, thread (i, connection): row i + 1 of dF/dXp (column 0 only) and
-// of dF/dXs of both ends, accumulated in shared memory in the reference's
-// order. Phase 2, thread (column, connection): that column of
-// dt (dF/dXp + dF/dXs dSec_dPri) (DaABpbC + Dscalar) for both ends, the sum
-// over k in order and the dF/dXp entry last, as dgemm with beta = 1 forms
-// it; stored as (row eId, col bId) = -bmatB and (row bId, col eId) = bmatE.
-template <int NCOM>
-__global__ void __launch_bounds__(ConnBlock<NCOM>::THREADS) k_conn_block(const ConnDev C, const ocpf_jac_bulk B,
-                                                                           const int32_t* up, const double* uprho,
-                                                                           double dt, ocpf_jac_out O)
+// |x| within 2^-200 .. 2^200, or zero: a product of two such values divided
+// by a third neither overflows nor loses bits to underflow on the way.
+__device__ __forceinline__ bool mid_range(double x)
 {
-    using CB = ConnBlock<NCOM>;
-    constexpr int NCOL = CB::NCOL, NSEC = CB::NSEC, CPB = CB::CPB;
-    extern __shared__ double sm[];
-    // rows[end][k][i][cl], prow[end][i][cl], then nsec[end][cl], ok[cl]
-    double* rows = sm;
-    double* prow = sm + (size_t)2 * NSEC * NCOM * CPB;
-    double* stg  = prow + (size_t)2 * NCOM * CPB;
-    int*    meta = (int*)(stg + (size_t)CB::STG * CPB);
-    // staged values: scalar v of phase j, derivative q (= 3 j1 + which) of
-    // phase j, partial w of phase j and component k
-    auto SC = [&](int j, int v, int cl) -> double& { return stg[(j * 11 + v) * CPB + cl]; };
-    auto PK = [&](int j, int q, int cl) -> double& { return stg[(33 + j * 9 + q) * CPB + cl]; };
-    auto CX = [&](int j, int k, int w, int cl) -> double& { return stg[(60 + (j * NCOM + k) * 5 + w) * CPB + cl]; };
-    auto R  = [&](int end, int k, int i, int cl) -> double& { return rows[((end * NSEC + k) * NCOM + i) * CPB + cl]; };
-    auto PR = [&](int end, int i, int cl) -> double& { return prow[(end * NCOM + i) * CPB + cl]; };
+    const uint32_t h = (uint32_t)__double2hiint(x) & 0x7fffffffu;
+    return (h - (823u << 20)) < (400u << 20) || x == 0;
+}
+
+__device__ __noinline__ double div_any(double a, double b) { return __ddiv_rn(a, b); }
+
+// q[i] = a[i] / b, correctly rounded, from y = RN(1 / b) (P. Markstein,
+// Computation of elementary functions on the IBM RISC System/6000 processor,
+// 1990): one correction makes q faithful, its residual is then exact, and
+// the second rounds correctly. All quotients by a phase's viscosity share y,
+// and nothing orders them against one another. `safe`: a, b and a / b are
+// away from the ends of the exponent range.
+template <int N>
+__device__ __forceinline__ void div_by(const double (&a)[N], double b, double y, bool safe, double (&q)[N])
+{
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        q[i] = M(a[i], y);
+        q[i] = __fma_rn(__fma_rn(-b, q[i], a[i]), y, q[i]);
+        q[i] = __fma_rn(__fma_rn(-b, q[i], a[i]), y, q[i]);
+    }
+    if (!safe)
+        for (int i = 0; i < N; i++) q[i] = div_any(a[i], b);
+}
+
+template <int NCOM>
+__device__ __forceinline__ void stage_phase(const ConnDev& C, const ocpf_jac_bulk& B, const int32_t* up,
+                                            const double* uprho, int64_t c, int j, int lane, ConnStage<NCOM>& sm)
+{
     const int64_t nc = C.nconn, nb = C.nb;
-    const int     lane_c = threadIdx.x % CPB, part = threadIdx.x / CPB;
-    for (int64_t g0 = (int64_t)blockIdx.x * CPB; g0 < nc; g0 += (int64_t)gridDim.x * CPB) {
-        const int64_t c     = g0 + lane_c;
-        const bool    live  = c < nc;
-        const int     i     = part;  // phase 1: row i + 1
-        __syncthreads();             // the previous group's phase 2 is done with the shared rows
-        if (i < NCOM) {
-            for (int k = 0; k < NSEC; k++) R(0, k, i, lane_c) = R(1, k, i, lane_c) = 0;
-            PR(0, i, lane_c) = PR(1, i, lane_c) = 0;
+    const int64_t bId = C.bId[c], eId = C.eId[c];
+    const int64_t u   = up[j * nc + c];
+    const bool    xb  = B.phaseExist[j * nb + bId] != 0, xe = B.phaseExist[j * nb + eId] != 0;
+    const uint32_t vB = B.pVnumCom[j * nb + bId], vE = B.pVnumCom[j * nb + eId];
+    uint32_t       f  = (u == bId ? F_UPB : 0u) | (xb ? F_EXB : 0u) | (xe ? F_EXE : 0u) |
+                 (B.pSderExist[j * nb + bId] != 0 ? F_SDB : 0u) | (B.pSderExist[j * nb + eId] != 0 ? F_SDE : 0u);
+    // shapes a flash writes: at most NCOM - 1 compositions per phase (and
+    // NSEC dSec_dPri rows, checked by the caller); anything else (and an
+    // upstream bulk that is neither end) gives NaN blocks
+    if ((u != bId && u != eId) || vB >= (uint32_t)NCOM || vE >= (uint32_t)NCOM)
+        f |= F_BAD;
+    else
+        f |= vB << 8 | vE << 16;
+    if (!(f & F_BAD) && (u == bId ? xb : xe)) {
+        f |= F_EXU;
+        for (int i = 0; i < NCOM; i++) copy8(&sm.x[j * NCOM + i][lane], B.xij + (int64_t)(j * NCOM + i) * nb + u);
+        const int64_t uj     = j * nb + u;
+        const double  Akd    = M(J_CONV1 * J_CONV2, C.area[c]);
+        const double  dGamma = M(J_GRAV, S(B.depth[bId], B.depth[eId]));
+        const double  mu = B.mu[uj], muP = B.muP[uj], t = M(Akd, B.kr[uj]);
+        const double  y  = __drcp_rn(mu);
+        if (mid_range(mu) && mu != 0 && mid_range(muP) && mid_range(t)) f |= F_SAFE;
+        sm.q[j][Q_DP][lane] = S(S(B.Pj[j * nb + bId], B.Pj[j * nb + eId]), M(uprho[j * nc + c], dGamma));
+        sm.q[j][Q_XI][lane]    = B.xi[uj];
+        sm.q[j][Q_MU][lane]    = mu;
+        sm.q[j][Q_Y][lane]     = y;
+        sm.q[j][Q_MUP][lane]   = muP;
+        sm.q[j][Q_XIP][lane]   = B.xiP[uj];
+        sm.q[j][Q_RHOP][lane]  = B.rhoP[uj];
+        sm.q[j][Q_RHOPB][lane] = xb ? B.rhoP[j * nb + bId] : 0.0;
+        sm.q[j][Q_RHOPE][lane] = xe ? B.rhoP[j * nb + eId] : 0.0;
+        const double num[1] = {t};
+        double       tr[1];
+        div_by(num, mu, y, (f & F_SAFE) != 0, tr);
+        sm.q[j][Q_TR][lane] = tr[0];
+    }
+    sm.f[j][lane] = f;
+}
+
+// Rows row0 .. row0 + NR - 1 (of the NCOM component rows; those before
+// `first` belong to the group before and are not stored) of one end's block: dF/dXp's column 0 and each dF/dXs entry in the reference's order,
+// every entry multiplied into the NCOL sums as soon as it is formed. `end`
+// is warp-uniform. The sum of an entry over k runs over the compact
+// dSec_dPri rows in order, the dF/dXp entry last, as dgemm with beta = 1
+// forms it; stored as (row eId, col bId) = -bmatB or (row bId, col eId) = bmatE.
+template <int NCOM>
+__device__ __forceinline__ void conn_rows(const ConnDev& C, const ocpf_jac_bulk& B, double dt,
+                                          const ocpf_jac_out& O, int64_t c, int lane, int end, int row0, int first,
+                                          const ConnStage<NCOM>& sm)
+{
+    using CT = ConnTile<NCOM>;
+    constexpr int NCOL = CT::NCOL, NR = CT::NR;
+    const int64_t nc = C.nconn, nb = C.nb;
+    const int64_t bId = C.bId[c], eId = C.eId[c];
+    const int64_t n      = end ? eId : bId;  // this end's bulk
+    const double  Akd    = M(J_CONV1 * J_CONV2, C.area[c]);
+    const double  dGamma = M(J_GRAV, S(B.depth[bId], B.depth[eId]));
+    const int     vsh    = end ? 16 : 8;
+    const uint32_t ex_me = end ? F_EXE : F_EXB, sd_me = end ? F_SDE : F_SDB;
+    uint32_t      fl[J_NP];
+    int           nsat = 0, ncomp = 0, noth = 0;
+    bool          ok = true, odd = false;
+#pragma unroll
+    for (int j = 0; j < J_NP; j++) {
+        fl[j] = sm.f[j][lane];
+        nsat += (fl[j] & sd_me) ? 1 : 0;
+        ncomp += (fl[j] >> vsh) & 0xff;
+        noth += ((fl[j] >> (24 - vsh)) & 0xff) + ((fl[j] & (end ? F_SDB : F_SDE)) ? 1 : 0);
+        ok  = ok && !(fl[j] & F_BAD);
+        // a phase of both bulks with different composition counts (no flash
+        // writes it): its columns can run into the next phase's
+        odd = odd || ((fl[j] & F_EXB) && (fl[j] & F_EXE) && ((fl[j] >> 8) & 0xff) != ((fl[j] >> 16) & 0xff));
+    }
+    ok = ok && nsat + ncomp <= CT::NSEC && noth <= CT::NSEC;
+    double* dst = (end ? O.offBE : O.offEB) + c;
+    if (!ok) {
+        for (int e = (row0 ? row0 + 1 : 0) * NCOL; e < (row0 + NR + 1) * NCOL; e++)
+            dst[(int64_t)e * nc] = __longlong_as_double(0x7ff8000000000000LL);
+        return;
+    }
+    if (row0 == 0) {
+#pragma unroll
+        for (int col = 0; col < NCOL; col++) dst[(int64_t)col * nc] = end ? M(0.0, dt) : -M(0.0, dt);
+    }
+    double acc[NR][NCOL], p[NR], rs[J_NP][NR];
+#pragma unroll
+    for (int i = 0; i < NR; i++) {
+        p[i] = 0;
+#pragma unroll
+        for (int col = 0; col < NCOL; col++) acc[i][col] = 0;
+#pragma unroll
+        for (int j1 = 0; j1 < J_NP; j1++) rs[j1][i] = 0;
+    }
+    // dF/dXp's column 0 and the saturation columns of dF/dXs
+    double dPc[J_NP][J_NP], dKr[J_NP][J_NP];
+#pragma unroll
+    for (int j = 0; j < J_NP; j++)
+#pragma unroll
+        for (int j1 = 0; j1 < J_NP; j1++) {
+            dPc[j][j1] = B.dPcj_dS[(int64_t)(3 * j + j1) * nb + n];
+            dKr[j][j1] = B.dKr_dS[(int64_t)(3 * j + j1) * nb + n];
         }
-        // phase 0: each connection's per-phase upstream data, once
-        if (live) {
-            const int64_t bId = C.bId[c], eId = C.eId[c];
-            const double  Akd    = M(J_CONV1 * J_CONV2, C.area[c]);
-            const double  dGamma = M(J_GRAV, S(B.depth[bId], B.depth[eId]));
-            for (int j = part; j < J_NP; j += CB::TPC) {
-                const int64_t u   = up[j * nc + c];
-                const bool    xb  = B.phaseExist[j * nb + bId] != 0, xe = B.phaseExist[j * nb + eId] != 0;
-                const bool    val = (u == bId || u == eId);
-                const bool    exU = val && (u == bId ? xb : xe);
-                SC(j, 10, lane_c) = exU ? 1.0 : 0.0;
-                if (exU) {
-                    const int64_t uj = j * nb + u;
-                    SC(j, 0, lane_c) = S(S(B.Pj[j * nb + bId], B.Pj[j * nb + eId]), M(uprho[j * nc + c], dGamma));
-                    SC(j, 1, lane_c) = B.xi[uj];
-                    SC(j, 2, lane_c) = B.kr[uj];
-                    SC(j, 3, lane_c) = B.mu[uj];
-                    SC(j, 4, lane_c) = B.muP[uj];
-                    SC(j, 5, lane_c) = B.xiP[uj];
-                    SC(j, 6, lane_c) = B.rhoP[uj];
-                    SC(j, 7, lane_c) = xb ? B.rhoP[j * nb + bId] : 0.0;
-                    SC(j, 8, lane_c) = xe ? B.rhoP[j * nb + eId] : 0.0;
-                    SC(j, 9, lane_c) = D(M(Akd, B.kr[uj]), B.mu[uj]);
-                }
-            }
-            for (int q = part; q < 9; q += CB::TPC) {
-                const int     j = q / 3, j1 = q % 3;
-                const int64_t u = up[j * nc + c];
-                const int64_t f = (int64_t)(3 * j + j1) * nb;
-                PK(j, 3 * j1 + 0, lane_c) = B.dPcj_dS[f + bId];
-                PK(j, 3 * j1 + 1, lane_c) = B.dPcj_dS[f + eId];
-                PK(j, 3 * j1 + 2, lane_c) = (u == bId || u == eId) ? B.dKr_dS[f + u] : 0.0;
-            }
-            for (int q = part; q < J_NP * NCOM; q += CB::TPC) {
-                const int     j = q / NCOM, k = q % NCOM;
-                const int64_t u = up[j * nc + c];
-                const int64_t f = (int64_t)(j * NCOM + k) * nb;
-                const bool    val = (u == bId || u == eId);
-                CX(j, k, 0, lane_c) = val ? B.rhox[f + u] : 0.0;
-                CX(j, k, 1, lane_c) = val ? B.xix[f + u] : 0.0;
-                CX(j, k, 2, lane_c) = val ? B.mux[f + u] : 0.0;
-                CX(j, k, 3, lane_c) = B.rhox[f + bId];
-                CX(j, k, 4, lane_c) = B.rhox[f + eId];
-            }
-        }
-        __syncthreads();
-        if (live && i < NCOM) {
-            const int64_t  bId = C.bId[c], eId = C.eId[c];
-            const double   Akd    = M(J_CONV1 * J_CONV2, C.area[c]);
-            const double   dGamma = M(J_GRAV, S(B.depth[bId], B.depth[eId]));
-            const SecShape sB = sec_shape(B, nb, bId), sE = sec_shape(B, nb, eId);
-            bool exB[J_NP], exE[J_NP];
 #pragma unroll
-            for (int j = 0; j < J_NP; j++) {
-                exB[j] = B.phaseExist[j * nb + bId] != 0;
-                exE[j] = B.phaseExist[j * nb + eId] != 0;
-            }
-            // shapes a flash writes: at most NCOM - 1 compositions per phase
-            // and NSEC dSec_dPri rows; anything else (and an upstream bulk
-            // that is neither end) gives NaN blocks instead of an access
-            // outside the arrays
-            bool ok = sB.ncol <= NSEC && sE.ncol <= NSEC;
+    for (int j = 0; j < J_NP; j++) {
+        const uint32_t f = fl[j];
+        if (!(f & F_EXU)) continue;
+        const bool    mine = ((f & F_UPB) != 0) == (end == 0);  // upstream is this end
+        const bool    both = (f & F_EXB) && (f & F_EXE);
+        const double  dP = sm.q[j][Q_DP][lane], xi = sm.q[j][Q_XI][lane], mu = sm.q[j][Q_MU][lane];
+        const double  y = sm.q[j][Q_Y][lane], muP = sm.q[j][Q_MUP][lane], tr = sm.q[j][Q_TR][lane];
+        const double  xiP  = sm.q[j][Q_XIP][lane];
+        const double  grho = M(-sm.q[j][Q_RHOP][lane], dGamma);
+        const double  gown = M(-sm.q[j][end ? Q_RHOPE : Q_RHOPB][lane], dGamma);
+        double tx[NR], a1[NR], a2[NR], dmu[NR], fk[NR];
+        bool   safe = (f & F_SAFE) != 0;
 #pragma unroll
-            for (int j = 0; j < J_NP; j++) {
-                ok = ok && sB.vn[j] >= 0 && sB.vn[j] < NCOM && sE.vn[j] >= 0 && sE.vn[j] < NCOM;
-                const int64_t u = up[j * nc + c];
-                ok = ok && (u == bId || u == eId);
-            }
-            if (i == 0) {
-                meta[lane_c]           = ok ? sB.ncol : 0;
-                meta[CPB + lane_c]     = ok ? sE.ncol : 0;
-                meta[2 * CPB + lane_c] = ok ? 1 : 0;
-            }
-            if (ok) {
-                double pB = 0, pE = 0;
-                int    jxB = (sB.sd[0] ? 1 : 0) + (sB.sd[1] ? 1 : 0) + (sB.sd[2] ? 1 : 0);
-                int    jxE = (sE.sd[0] ? 1 : 0) + (sE.sd[1] ? 1 : 0) + (sE.sd[2] ? 1 : 0);
-                for (int j = 0; j < J_NP; j++) {
-                    const int64_t uId = up[j * nc + c];
-                    const bool    exU = SC(j, 10, lane_c) != 0;
-                    if (!exU) {
-                        jxB += sB.vn[j];
-                        jxE += sE.vn[j];
-                        continue;
-                    }
-                    const double dP = SC(j, 0, lane_c), xi = SC(j, 1, lane_c), mu = SC(j, 3, lane_c);
-                    const double muP = SC(j, 4, lane_c), xiP = SC(j, 5, lane_c), rhoP = SC(j, 6, lane_c);
-                    const double transJ  = SC(j, 9, lane_c);
-                    const double xij     = B.xij[(int64_t)(j * NCOM + i) * nb + uId];
-                    const double transIJ = M(M(xij, xi), transJ);
-                    pB = A(pB, transIJ);
-                    pE = S(pE, transIJ);
-                    double tmp = M(M(M(xij, transJ), xiP), dP);
-                    tmp        = A(tmp, M(D(M(-transIJ, muP), mu), dP));
-                    if (!exE[j]) {
-                        tmp = A(tmp, M(transIJ, M(-rhoP, dGamma)));
-                        pB  = A(pB, tmp);
-                    } else if (!exB[j]) {
-                        tmp = A(tmp, M(transIJ, M(-rhoP, dGamma)));
-                        pE  = A(pE, tmp);
-                    } else {
-                        pB = A(pB, M(M(transIJ, M(-SC(j, 7, lane_c), dGamma)), 0.5));
-                        pE = A(pE, M(M(transIJ, M(-SC(j, 8, lane_c), dGamma)), 0.5));
-                        if (bId == uId)
-                            pB = A(pB, tmp);
-                        else
-                            pE = A(pE, tmp);
-                    }
-                    int          j1SB = 0, j1SE = 0;
-                    const double fk   = D(M(M(Akd, xij), xi), mu);  // Akd xij xi / mu
-                    if (bId == uId) {
+        for (int i = 0; i < NR; i++) {
+            const double xij = sm.x[j * NCOM + row0 + i][lane];
+            tx[i] = M(M(xij, xi), tr);
+            a1[i] = M(M(Akd, xij), xi);
+            a2[i] = M(-tx[i], muP);
+            safe  = safe && mid_range(tx[i]) && mid_range(a1[i]);
+            p[i]  = end ? S(p[i], tx[i]) : A(p[i], tx[i]);
+            if (both) p[i] = A(p[i], M(M(tx[i], gown), 0.5));
 #pragma unroll
-                        for (int j1 = 0; j1 < J_NP; j1++) {
-                            if (sB.sd[j1]) {
-                                double& r = R(0, j1SB, i, lane_c);
-                                r         = A(r, M(transIJ, PK(j, 3 * j1 + 0, lane_c)));
-                                r         = A(r, M(M(fk, PK(j, 3 * j1 + 2, lane_c)), dP));
-                                j1SB++;
-                            }
-                            if (sE.sd[j1]) {
-                                double& r = R(1, j1SE, i, lane_c);
-                                r         = S(r, M(transIJ, PK(j, 3 * j1 + 1, lane_c)));
-                                j1SE++;
-                            }
-                        }
-                        const int nv = sB.vn[j];
-#pragma unroll
-                        for (int k = 0; k < NCOM - 1; k++) {
-                            if (k >= nv) break;
-                            const double rx = exE[j] ? M(CX(j, k, 3, lane_c), 0.5) : CX(j, k, 0, lane_c);
-                            double       v  = M(M(-transIJ, rx), dGamma);
-                            v               = A(v, M(M(M(xij, transJ), CX(j, k, 1, lane_c)), dP));
-                            v               = A(v, M(D(M(-transIJ, CX(j, k, 2, lane_c)), mu), dP));
-                            double& r       = R(0, jxB + k, i, lane_c);
-                            r               = A(r, v);
-                            if (exE[j]) {
-                                double& re = R(1, jxE + k, i, lane_c);
-                                re         = A(re, M(M(M(-transIJ, CX(j, k, 4, lane_c)), 0.5), dGamma));
-                            }
-                        }
-                        if (i < nv) {
-                            double& r = R(0, jxB + i, i, lane_c);
-                            r         = A(r, M(M(xi, transJ), dP));
-                        }
-                    } else {
-#pragma unroll
-                        for (int j1 = 0; j1 < J_NP; j1++) {
-                            if (sB.sd[j1]) {
-                                double& r = R(0, j1SB, i, lane_c);
-                                r         = A(r, M(transIJ, PK(j, 3 * j1 + 0, lane_c)));
-                                j1SB++;
-                            }
-                            if (sE.sd[j1]) {
-                                double& r = R(1, j1SE, i, lane_c);
-                                r         = S(r, M(transIJ, PK(j, 3 * j1 + 1, lane_c)));
-                                r         = A(r, M(M(fk, PK(j, 3 * j1 + 2, lane_c)), dP));
-                                j1SE++;
-                            }
-                        }
-                        const int nv = sE.vn[j];
-#pragma unroll
-                        for (int k = 0; k < NCOM - 1; k++) {
-                            if (k >= nv) break;
-                            const double rx = exB[j] ? M(CX(j, k, 4, lane_c), 0.5) : CX(j, k, 0, lane_c);
-                            double       v  = M(M(-transIJ, rx), dGamma);
-                            v               = A(v, M(M(M(xij, transJ), CX(j, k, 1, lane_c)), dP));
-                            v               = A(v, M(D(M(-transIJ, CX(j, k, 2, lane_c)), mu), dP));
-                            double& r       = R(1, jxE + k, i, lane_c);
-                            r               = A(r, v);
-                            if (exB[j]) {
-                                double& rb = R(0, jxB + k, i, lane_c);
-                                rb         = A(rb, M(M(M(-transIJ, CX(j, k, 3, lane_c)), 0.5), dGamma));
-                            }
-                        }
-                        if (i < nv) {
-                            double& r = R(1, jxE + i, i, lane_c);
-                            r         = A(r, M(M(xi, transJ), dP));
-                        }
-                    }
-                    jxB += sB.vn[j];
-                    jxE += sE.vn[j];
-                }
-                PR(0, i, lane_c) = pB;
-                PR(1, i, lane_c) = pE;
+            for (int j1 = 0; j1 < J_NP; j1++) {
+                const double t = M(tx[i], dPc[j][j1]);
+                rs[j1][i]      = end ? S(rs[j1][i], t) : A(rs[j1][i], t);
             }
         }
-        __syncthreads();
-        const int col = part;  // phase 2: column col
-        if (live && col < NCOL) {
-            const int64_t bId = C.bId[c], eId = C.eId[c];
-            const bool    ok  = meta[2 * CPB + lane_c] != 0;
-            const double  nan = __longlong_as_double(0x7ff8000000000000LL);
-            for (int end = 0; end < 2; end++) {
-                const int64_t n    = end ? eId : bId;
-                const int     nsec = meta[end * CPB + lane_c];
-                double*       dst  = end ? O.offBE : O.offEB;
-                dst[(int64_t)col * nc + c] = !ok ? nan : (end ? M(0.0, dt) : -M(0.0, dt));  // row 0
-                double sec[NSEC];
+        if (mine) {
+            div_by(a2, mu, y, safe, dmu);
+            div_by(a1, mu, y, safe, fk);
 #pragma unroll
-                for (int k = 0; k < NSEC; k++) sec[k] = k < nsec ? B.dSec_dPri[(int64_t)(k * NCOL + col) * nb + n] : 0.0;
+            for (int i = 0; i < NR; i++) {
+                double tmp = M(M(M(sm.x[j * NCOM + row0 + i][lane], tr), xiP), dP);
+                tmp        = A(tmp, M(dmu[i], dP));
+                if (!both) tmp = A(tmp, M(tx[i], grho));
+                p[i] = A(p[i], tmp);
 #pragma unroll
-                for (int r = 1; r <= NCOM; r++) {
-                    double v = nan;
-                    if (ok) {
-                        double s2 = 0;
-#pragma unroll
-                        for (int k = 0; k < NSEC; k++)
-                            if (k < nsec) s2 = A(s2, M(R(end, k, r - 1, lane_c), sec[k]));
-                        v = M(A(s2, col == 0 ? PR(end, r - 1, lane_c) : 0.0), dt);
-                        if (!end) v = -v;
-                    }
-                    dst[(int64_t)(r * NCOL + col) * nc + c] = v;
-                }
+                for (int j1 = 0; j1 < J_NP; j1++) rs[j1][i] = A(rs[j1][i], M(M(fk[i], dKr[j][j1]), dP));
             }
         }
     }
+    // compact row k, column col: sec[(k NCOL + col) step]
+    const double* sec  = CT::STAGED ? sm.sec + (size_t)end * CT::NENT * 32 + lane : B.dSec_dPri + n;
+    const int64_t step = CT::STAGED ? 32 : nb;
+    auto product = [&](const double (&r)[NR]) {
+        double s[NCOL];
+#pragma unroll
+        for (int col = 0; col < NCOL; col++) {
+            s[col] = *sec;
+            sec += step;
+        }
+#pragma unroll
+        for (int i = 0; i < NR; i++)
+#pragma unroll
+            for (int col = 0; col < NCOL; col++) acc[i][col] = A(acc[i][col], M(r[i], s[col]));
+    };
+#pragma unroll
+    for (int j1 = 0; j1 < J_NP; j1++)
+        if (fl[j1] & sd_me) product(rs[j1]);
+    // the composition columns: those of phase j follow those of phase j - 1.
+    // Entry (i, kk) of phase j at this end, or 0
+    auto comp_load = [&](int j, int kk, double (&v)[3]) {
+        const int64_t q = (int64_t)(j * NCOM + kk) * nb + n;
+        v[0] = B.rhox[q], v[1] = B.xix[q], v[2] = B.mux[q];
+    };
+    auto comp_entry = [&](int j, uint32_t f, int kk, const double (&part)[3], double (&r)[NR]) {
+        const bool    mine = ((f & F_UPB) != 0) == (end == 0);
+        const bool    both = (f & F_EXB) && (f & F_EXE);
+        const double  xi = sm.q[j][Q_XI][lane], tr = sm.q[j][Q_TR][lane];
+        const double  rh = both ? M(part[0], 0.5) : part[0];
+        double        tx[NR], v[NR];
+        bool          safe = (f & F_SAFE) && mid_range(part[2]);
+#pragma unroll
+        for (int i = 0; i < NR; i++) {
+            tx[i] = M(M(sm.x[j * NCOM + row0 + i][lane], xi), tr);
+            safe  = safe && mid_range(tx[i]);
+            v[i]  = M(M(-tx[i], rh), dGamma);
+        }
+        if (mine) {
+            const double mu = sm.q[j][Q_MU][lane], y = sm.q[j][Q_Y][lane], dP = sm.q[j][Q_DP][lane];
+            const double own = M(M(xi, tr), dP);
+            double       num[NR], dmu[NR];
+#pragma unroll
+            for (int i = 0; i < NR; i++) num[i] = M(-tx[i], part[2]);
+            div_by(num, mu, y, safe, dmu);
+#pragma unroll
+            for (int i = 0; i < NR; i++) {
+                v[i] = A(v[i], M(M(M(sm.x[j * NCOM + row0 + i][lane], tr), part[1]), dP));
+                v[i] = A(v[i], M(dmu[i], dP));
+                r[i] = A(r[i], v[i]);
+                if (row0 + i == kk) r[i] = A(r[i], own);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < NR; i++) r[i] = A(r[i], v[i]);
+        }
+    };
+    if (!odd) {
+#pragma unroll 1
+        for (int j = 0; j < J_NP; j++) {
+            const uint32_t f  = sm.f[j][lane];
+            const int      nv = (f >> vsh) & 0xff;
+            const bool     on = (f & F_EXU) && ((((f & F_UPB) != 0) == (end == 0)) || (f & ex_me));
+            double         next[3] = {0, 0, 0};
+            if (on && nv > 0) comp_load(j, 0, next);
+#pragma unroll 1
+            for (int kk = 0; kk < nv; kk++) {
+                double       r[NR];
+                const double part[3] = {next[0], next[1], next[2]};
+#pragma unroll
+                for (int i = 0; i < NR; i++) r[i] = 0;
+                if (on) {
+                    if (kk + 1 < nv) comp_load(j, kk + 1, next);
+                    comp_entry(j, f, kk, part, r);
+                }
+                product(r);
+            }
+        }
+    } else {
+        // every column gathers what each phase's run of columns leaves in it
+#pragma unroll 1
+        for (int k = nsat; k < nsat + ncomp; k++) {
+            double r[NR];
+            int    j0 = nsat;
+#pragma unroll
+            for (int i = 0; i < NR; i++) r[i] = 0;
+#pragma unroll 1
+            for (int j = 0; j < J_NP; j++) {
+                const uint32_t f    = sm.f[j][lane];
+                const bool     mine = ((f & F_UPB) != 0) == (end == 0);
+                const int      cnt  = (f >> (mine ? vsh : 24 - vsh)) & 0xff;
+                if ((f & F_EXU) && (mine || (f & ex_me)) && k >= j0 && k < j0 + cnt) {
+                    double part[3];
+                    comp_load(j, k - j0, part);
+                    comp_entry(j, f, k - j0, part, r);
+                }
+                j0 += (f >> vsh) & 0xff;
+            }
+            product(r);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < NR; i++) {
+        if (row0 + i < first) continue;  // the group before has it
+        double* d = dst + (int64_t)(row0 + i + 1) * NCOL * nc;
+#pragma unroll
+        for (int col = 0; col < NCOL; col++) {
+            const double v = M(A(acc[i][col], col == 0 ? p[i] : 0.0), dt);
+            *d             = end ? v : -v;
+            d += nc;
+        }
+    }
+}
+
+template <int NCOM>
+__global__ void __launch_bounds__(ConnTile<NCOM>::THREADS, ConnTile<NCOM>::MINB)
+    k_conn_block(const __grid_constant__ ConnDev C, const __grid_constant__ ocpf_jac_bulk B, const int32_t* up,
+                 const double* uprho, double dt, const __grid_constant__ ocpf_jac_out O)
+{
+    using CT = ConnTile<NCOM>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ConnStage<NCOM>* stage = reinterpret_cast<ConnStage<NCOM>*>(smem_raw);
+    const int     tile = threadIdx.x / CT::TPT, w = (threadIdx.x % CT::TPT) >> 5, lane = threadIdx.x & 31;
+    const int64_t c    = ((int64_t)blockIdx.x * CT::TILES + tile) * 32 + lane;
+    const bool    live = c < C.nconn;
+    const int     end = w & 1, g = w >> 1;
+    if (live) {
+        if (CT::STAGED) {
+            // this end's rows; as many as the bulk has
+            const int64_t nb = C.nb, n = end ? C.eId[c] : C.bId[c];
+            int           rows = 0;
+#pragma unroll
+            for (int j = 0; j < J_NP; j++)
+                rows += min((int)(B.pVnumCom[j * nb + n] & 0xff), NCOM) + (B.pSderExist[j * nb + n] ? 1 : 0);
+            const int     cnt = min(rows, CT::NSEC) * CT::NCOL;
+            double*       d   = stage[tile].sec + (size_t)end * CT::NENT * 32 + lane;
+            const double* s   = B.dSec_dPri + n;
+#pragma unroll 4
+            for (int e = g; e < cnt; e += CT::G) copy8(d + e * 32, s + (int64_t)e * nb);
+        }
+        for (int j = w; j < J_NP; j += 2 * CT::G) stage_phase<NCOM>(C, B, up, uprho, c, j, lane, stage[tile]);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (!live) return;
+    conn_rows<NCOM>(C, B, dt, O, c, lane, end, min(g * CT::NR, NCOM - CT::NR), g * CT::NR, stage[tile]);
 }
 
 template <int NCOM>
@@ -408,13 +494,14 @@ template <int NCOM>
 cudaError_t launch_jac(const ConnDev& C, const ocpf_jac_bulk& B, const int32_t* up, const double* uprho, double dt,
                        const ocpf_jac_out& O, int sms, cudaStream_t st)
 {
-    using CB = ConnBlock<NCOM>;
-    // per device; cheap, so on every launch
-    cudaFuncSetAttribute(k_conn_block<NCOM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CB::SMEM);
+    using CT = ConnTile<NCOM>;
     const int64_t t2 = (NCOM + 1) * C.nb;
-    const int     g1 = (int)std::min<int64_t>((C.nconn + CB::CPB - 1) / CB::CPB, (int64_t)sms * 8);
+    const int64_t g1 = (C.nconn + 32 * CT::TILES - 1) / (32 * CT::TILES);  // < 2^31: at most 2^30 connections
     const int     g2 = (int)std::min<int64_t>((t2 + 127) / 128, (int64_t)sms * 16);
-    if (C.nconn > 0) k_conn_block<NCOM><<<g1, CB::THREADS, CB::SMEM, st>>>(C, B, up, uprho, dt, O);
+    const int     smem = (int)sizeof(ConnStage<NCOM>) * CT::TILES;
+    // per device; cheap, so on every launch
+    cudaFuncSetAttribute(k_conn_block<NCOM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (C.nconn > 0) k_conn_block<NCOM><<<(unsigned)g1, CT::THREADS, smem, st>>>(C, B, up, uprho, dt, O);
     if (C.nb > 0) k_diag_rows<NCOM><<<g2, 128, 0, st>>>(C, B, O);
     return cudaGetLastError();
 }
