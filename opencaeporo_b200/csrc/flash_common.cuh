@@ -32,15 +32,15 @@ constexpr double D1TD2        = D1 * D2;
 // J.-M. Muller et al., Handbook of Floating-Point Arithmetic, 2nd ed., 2018,
 // ch. 4). Three dependent FP64 operations in place of a division, with the
 // same result bits. Zeros, non-finite values and magnitudes outside
-// [1e-270, 1e270] (where r or r rd could leave the normal range) take the
-// ordinary division.
+// [2^-896, 2^896) (where r or r rd could leave the normal range) take the
+// ordinary division, tested after the quotient is on its way.
 __device__ __forceinline__ double div_const(double x, double d, double rd)
 {
-    const double ax = fabs(x);
-    if (!(ax > 1e-270 && ax < 1e270)) return x / d;
-    const double q = x * rd;
-    const double r = fma(-d, q, x);
-    return fma(r, rd, q);
+    const double   q0 = __dmul_rn(x, rd);
+    double         q  = __fma_rn(__fma_rn(-d, q0, x), rd, q0);
+    const uint32_t h  = (uint32_t)__double2hiint(x) & 0x7fffffffu;
+    if (__builtin_expect(h - (127u << 20) >= (1792u << 20), 0)) q = x / d;
+    return q;
 }
 constexpr double RCP3     = 1.0 / 3;
 constexpr double RCP9     = 1.0 / 9;

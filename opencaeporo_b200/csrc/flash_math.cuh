@@ -4,11 +4,14 @@
 #pragma once
 
 #include "flash_common.cuh"
+#include "flash_div.cuh"
 
 namespace ocpf {
 
 // Newton polish of one cubic root, keeping the best iterate
-// (NTcubicroot, src/MixtureComp.cpp:5078-5102).
+// (NTcubicroot, src/MixtureComp.cpp:5078-5102). LAT: the division written for
+// latency (div1), for one cell's chain on a warp; the same value.
+template <bool LAT = false>
 __device__ __forceinline__ double nt_polish(double root, double a, double b, double c)
 {
     double e       = root * (root * (root + a) + b) + c;
@@ -17,7 +20,7 @@ __device__ __forceinline__ double nt_polish(double root, double a, double b, dou
     int    iter    = 0;
     while (fabs(e) > 1e-8) {
         const double df = root * (3 * root + 2 * a) + b;
-        root            = root - e / df;
+        root            = root - (LAT ? div1(e, df) : e / df);
         iter++;
         if (iter > 10) break;
         e = root * (root * (root + a) + b) + c;
@@ -54,6 +57,14 @@ struct PrCubic {
         const double a3  = div_const(a, 3, RCP3);
         const double arg = div_const(k == 1 ? theta + 2 * PI_TRUNC : (k == 2 ? theta - 2 * PI_TRUNC : theta), 3, RCP3);
         return nt_polish(s2 * cos(arg) - a3, a, b, c);
+    }
+    // trig_root for lanes that polish different roots, sqrt(Q) given
+    __device__ __forceinline__ double trig_root_lane(int k, double theta, double sqrtQ) const
+    {
+        const double s2  = -2 * sqrtQ;
+        const double a3  = div_const(a, 3, RCP3);
+        const double arg = div_const(theta + (k == 1 ? 2 * PI_TRUNC : (k == 2 ? -2 * PI_TRUNC : 0.0)), 3, RCP3);
+        return nt_polish<true>(s2 * cos(arg) - a3, a, b, c);
     }
     // The single real root (M > 0), polished.
     __device__ __forceinline__ double cardano_root() const
@@ -113,6 +124,37 @@ __device__ __forceinline__ double sol_eos(double aj, double bj)
     } else {
         return cu.cardano_root();
     }
+}
+
+// The roots sol_eos chooses between, for a group of lanes that all hold the
+// same (aj, bj): zmin and zmax, the smallest and largest of three real roots
+// (returns true), or both the single real root (returns false), on every
+// lane of `mask`. The group has 16 lanes from `base`; its lanes 0, 1 and 2 each polish
+// one of the three trigonometric roots; even and odd lanes form one cube root
+// each of Cardano's form. Same values as sol_eos, bit for bit.
+__device__ __forceinline__ bool root_pair_group(double aj, double bj, unsigned mask, int base, int rank, double& zmin,
+                                                double& zmax)
+{
+    const PrCubic cu(aj, bj);
+    if (cu.M <= 0) {
+        // both square roots at once, on different lanes
+        const double rt    = sqrt((rank & 8) ? cu.Q : cu.Q3);
+        const double theta = acos(div1(cu.R, __shfl_sync(mask, rt, base)));
+        const double zk    = cu.trig_root_lane(rank < 3 ? rank : 0, theta, __shfl_sync(mask, rt, base + 8));
+        const double z0    = __shfl_sync(mask, zk, base);
+        const double z1    = __shfl_sync(mask, zk, base + 1);
+        const double z2    = __shfl_sync(mask, zk, base + 2);
+        zmin               = fmin(z0, fmin(z1, z2));
+        zmax               = fmax(z0, fmax(z1, z2));
+        return true;
+    }
+    const double sM   = sqrt(cu.M);
+    const double t    = ((rank & 1) ? cu.R : -cu.R) + sM;
+    const double st   = signD(t) * cbrt(fabs(t));
+    const double S    = __shfl_sync(mask, st, base);
+    const double T    = -__shfl_sync(mask, st, base + 1);
+    zmin = zmax       = nt_polish<true>(S + T - div_const(cu.a, 3, RCP3), cu.a, cu.b, cu.c);
+    return false;
 }
 
 // sol_eos for a group of lanes that all hold the same (aj, bj): lanes
