@@ -128,6 +128,12 @@ struct Lists {
     }
     __device__ __forceinline__ uint32_t len(int id) const { return *(volatile uint32_t*)&ctr[2 * id]; }
     __device__ __forceinline__ int32_t item(int id, uint32_t k) const { return items[(int64_t)id * cap + k]; }
+    // next item of list `id` for a second consumer, counted on list `head`
+    __device__ __forceinline__ int32_t take_again(int id, int head, uint32_t n) const
+    {
+        const uint32_t k = atomicAdd(&ctr[2 * head + 1], 1u);
+        return k < n ? item(id, k) : -1;
+    }
     // next item for a persistent consumer, or -1
     __device__ __forceinline__ int32_t take(int id, uint32_t n) const
     {

@@ -20,6 +20,9 @@
 namespace ocpf {
 
 constexpr int kNC = OCPF_NC;
+// The split's iterations partly on whole warps: where the results keep their
+// bits (beyond 6 components the compiler rounds the two forms differently).
+constexpr bool kSplitWarp = kNC <= 6;
 
 #define K128 __global__ void __launch_bounds__(128)
 K128 KP(init)(const __grid_constant__ FluidConst F, const PhasedArgs a) { init_body<kNC>(F, a); }
@@ -39,7 +42,14 @@ K128 KP(sta_nr)(const __grid_constant__ FluidConst F, const PhasedArgs a, int k,
     sta_nr_body<kNC>(F, a, k, list, fallback);
 }
 K128 KP(sp_prep)(const __grid_constant__ FluidConst F, const PhasedArgs a, int r) { sp_prep_body<kNC>(F, a, r); }
-K128 KP(sp_ssm)(const __grid_constant__ FluidConst F, const PhasedArgs a, int r) { sp_ssm_body<kNC>(F, a, r); }
+K128 KP(sp_ssm)(const __grid_constant__ FluidConst F, const PhasedArgs a, int r, uint32_t park)
+{
+    sp_ssm_body<kNC>(F, a, r, park);
+}
+__global__ void __launch_bounds__(128, 4) KP(sp_ssm_warp)(const __grid_constant__ FluidConst F, const PhasedArgs a, int r)
+{
+    sp_ssm_warp_body<kNC>(F, a, r);
+}
 K128 KP(sp_nrinit)(const __grid_constant__ FluidConst F, const PhasedArgs a, int r) { sp_nrinit_body<kNC>(F, a, r); }
 K128 KP(sp_nr)(const __grid_constant__ FluidConst F, const PhasedArgs a, int r) { sp_nr_body<kNC>(F, a, r); }
 K128 KP(slow)(const __grid_constant__ FluidConst F, const PhasedArgs a, int list) { slow_body<kNC>(F, a, list); }
@@ -72,12 +82,17 @@ int OCPF_CAT(persistent_grid_, OCPF_NC)(const void* k, int sms, int pct)
     return sms * use;
 }
 
-// One split round: set-up, successive substitution, Newton start, Newton.
+// One split round: set-up, successive substitution, Newton.
 void OCPF_CAT(split_round_, OCPF_NC)(const FluidConst& F, const PhasedArgs& a, cudaStream_t st, int r, int gp,
-                                    int bp, int gs, int gnr)
+                                    int bp, int gs, int gnr, int gw)
 {
     KP(sp_prep)<<<gp, bp, 0, st>>>(F, a, r);
-    KP(sp_ssm)<<<gs, 128, 0, st>>>(F, a, r);
+    if constexpr (kSplitWarp) {
+        KP(sp_ssm)<<<gs, 128, 0, st>>>(F, a, r, 4u * (uint32_t)gw);
+        KP(sp_ssm_warp)<<<gw, 128, 0, st>>>(F, a, r);
+    } else {
+        KP(sp_ssm)<<<gs, 128, 0, st>>>(F, a, r, 0u);
+    }
     KP(sp_nrinit)<<<gp, bp, 0, st>>>(F, a, r);
     KP(sp_nr)<<<gnr, 128, 0, st>>>(F, a, r);
 }
@@ -126,7 +141,7 @@ cudaError_t OCPF_CAT(launch_phased_nc, OCPF_NC)(const FluidConst& F, const Phase
         // (with PH_DEFER their split waits until trial 1 has run, below)
         const int gl = (int)std::min<int64_t>((a.count + LEARN_TILE - 1) / LEARN_TILE, (int64_t)sms * 4);
         KP(learn)<<<gl, 128, sizeof(LearnSmem), st>>>(F, a);
-        if (!defer) OCPF_CAT(split_round_, OCPF_NC)(F, a, st, LEARN_ROUND, gp, bp, g_sp, g_spnr);
+        if (!defer) OCPF_CAT(split_round_, OCPF_NC)(F, a, st, LEARN_ROUND, gp, bp, g_sp, g_spnr, sms * 4);
     }
     for (int k = 0; k < 2; k++) {
         KP(s01_prep)<<<gp, bp, 0, st>>>(F, a, k);
@@ -165,7 +180,7 @@ cudaError_t OCPF_CAT(launch_phased_nc, OCPF_NC)(const FluidConst& F, const Phase
                 cudaEventRecord(side->fork[k], st);
                 cudaStreamWaitEvent(ss, side->fork[k], 0);
             }
-            OCPF_CAT(split_round_, OCPF_NC)(F, a, ss, TRIAL_ROUND0 + k, gp, bp, g_sp, g_spnr);
+            OCPF_CAT(split_round_, OCPF_NC)(F, a, ss, TRIAL_ROUND0 + k, gp, bp, g_sp, g_spnr, sms * 4);
             if (t.slow_threads)
                 KP(slow_thread)<<<gp, bp, 0, ss>>>(F, a, L_SLOW_T0 + k);
             else
@@ -184,7 +199,7 @@ cudaError_t OCPF_CAT(launch_phased_nc, OCPF_NC)(const FluidConst& F, const Phase
                 cudaEventRecord(side->fork[0], st);
                 cudaStreamWaitEvent(ss, side->fork[0], 0);
             }
-            OCPF_CAT(split_round_, OCPF_NC)(F, a, ss, LEARN_ROUND, gp, bp, g_sp, g_spnr);
+            OCPF_CAT(split_round_, OCPF_NC)(F, a, ss, LEARN_ROUND, gp, bp, g_sp, g_spnr, sms * 4);
             PhasedArgs b = a;
             b.sdup       = 1;
             b.opts &= ~(PH_EARLY | PH_DEFER);
@@ -193,7 +208,7 @@ cudaError_t OCPF_CAT(launch_phased_nc, OCPF_NC)(const FluidConst& F, const Phase
         }
     }
     if (defer && side) cudaStreamWaitEvent(st, side->join[0], 0);
-    for (int r = 0; r < SPLIT_ROUNDS; r++) OCPF_CAT(split_round_, OCPF_NC)(F, a, st, r, gp, bp, g_sp, g_spnr);
+    for (int r = 0; r < SPLIT_ROUNDS; r++) OCPF_CAT(split_round_, OCPF_NC)(F, a, st, r, gp, bp, g_sp, g_spnr, sms * 4);
     if (marks) cudaEventRecord(marks[0], st);
     if (t.slow_threads)
         KP(slow_thread)<<<gp, bp, 0, st>>>(F, a, L_SLOW);

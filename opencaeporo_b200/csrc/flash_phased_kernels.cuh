@@ -544,11 +544,71 @@ __device__ void sp_prep_body(const FluidConst& F, const PhasedArgs& a, int r)
     }
 }
 
+// The end of SplitSSM2's iterations for cell c, stored for the Newton start.
+template <int NC>
+__device__ __forceinline__ void sp_ssm_store(const CellFlash<NC>& f, const StateBuf& S, int64_t c, double Se, int iter,
+                                             bool cap)
+{
+    using F_ = SF<NC>;
+    if (cap) S.I(IF_META, c) &= ~(int32_t)M_C_SSMSP;
+    S.D(F_::SeSP, c) = Se;
+    S.I(IF_IT2, c) += iter;
+    S.I(IF_IT4, c) += f.it_rr;
+#pragma unroll
+    for (int i = 0; i < NC; i++) S.D(F_::Ks + i, c) = f.Ks[i];
+    store_split(f, S, c);
+}
+
+// Split lists of at most SSM_SMALL cells per warp of the whole-warp kernel go
+// to it at once; of longer ones it finishes what a warp of the one-lane kernel
+// is left with when the list is used up and it holds at most SSM_TAIL cells.
+// One lane takes 7 us a step (6 components; its warp's other lanes idle or in
+// other branches), the whole warp 2.6 us.
+constexpr int SSM_SMALL = 2, SSM_TAIL = 3;
+
+// SplitSSM2's iterations with one warp per cell (flash_warp.cuh), for the
+// cells of list L_SP_r when it is short, else for those the one-lane kernel
+// left on L_SPNR_r. `warps`: this kernel's whole grid.
+template <int NC>
+__device__ __noinline__ void sp_ssm_on_warp(const FluidConst& F, const PhasedArgs& a, int64_t c)
+{
+    using F_ = SF<NC>;
+    const StateBuf& S = a.S;
+    CellFlash<NC>   f(F);
+    f.P = a.in.P[c];
+    load_z<NC>(a, c, f.zi);
+#pragma unroll
+    for (int i = 0; i < NC; i++) {
+        f.Ks[i] = S.D(F_::Ks + i, c);
+        f.sA[i] = S.D(F_::sA + i, c);
+        f.Bi[i] = S.D(F_::Bi + i, c);
+    }
+    f.it_rr         = 0;
+    f.ssmsp_conflag = true;
+    f.nu[0]         = 0;
+    WarpSplit<NC> w(f);
+    int           iter = 0;
+    const double  Se   = w.ssm_steps(HUGE_VAL, S.D(F_::Stol, c), S.I(IF_MAXIT, c), iter);
+    if ((threadIdx.x & 31) == 0) sp_ssm_store(f, S, c, Se, iter, !f.ssmsp_conflag);
+    __syncwarp();
+}
+template <int NC>
+__device__ void sp_ssm_warp_body(const FluidConst& F, const PhasedArgs& a, int r)
+{
+    const uint32_t nw   = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t all  = a.L.len(L_SP_0 + r);
+    const int      list = all <= SSM_SMALL * nw ? L_SP_0 + r : L_SPNR_0 + r;
+    const uint32_t n    = a.L.len(list);
+    for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < n; k += nw)
+        sp_ssm_on_warp<NC>(F, a, a.L.item(list, k));
+}
+
 // SplitSSM2's iterations (src/MixtureComp.cpp:1881-1902) on a persistent
 // grid: per turn, Rachford-Rice, the phase compositions, the fugacities of
-// both phases, and the K update.
+// both phases, and the K update. With `park` (the warps of the whole-warp
+// kernel that follows; 0: none) short lists and tails are left to it.
 template <int NC>
-__device__ void sp_ssm_body(const FluidConst& F, const PhasedArgs& a, int r)
+__device__ void sp_ssm_body(const FluidConst& F, const PhasedArgs& a, int r, uint32_t park = 0)
 {
     using F_ = SF<NC>;
     const StateBuf& S    = a.S;
@@ -557,6 +617,7 @@ __device__ void sp_ssm_body(const FluidConst& F, const PhasedArgs& a, int r)
     CellFlash<NC>   f(F);  // holds z, K, x, phi, nu, Aj/Bj/Zj, sA, Bi
     double          Stol = 0;
     int             maxIt = 0, iter = 0;
+    if (n <= SSM_SMALL * park) return;
     int64_t         c     = a.L.take(list, n);
     auto load = [&]() {
         f.P = a.in.P[c];
@@ -574,7 +635,21 @@ __device__ void sp_ssm_body(const FluidConst& F, const PhasedArgs& a, int r)
         f.NP     = 2;
     };
     if (c >= 0) load();
-    while (__any_sync(0xffffffffu, c >= 0)) {
+    while (true) {
+        const uint32_t held = __ballot_sync(0xffffffffu, c >= 0);
+        if (held == 0) break;
+        if (park && __popc(held) <= SSM_TAIL) {
+            // lanes without a cell found the list used up
+            if (c >= 0) {
+#pragma unroll
+                for (int i = 0; i < NC; i++) S.D(F_::Ks + i, c) = f.Ks[i];
+                S.I(IF_IT2, c) += iter;
+                S.I(IF_IT4, c) += f.it_rr;
+                S.I(IF_MAXIT, c) = maxIt - iter;
+                a.L.push(L_SPNR_0 + r, (int32_t)c);
+            }
+            break;
+        }
         if (c >= 0) {
             f.rachford_rice2();
 #pragma unroll
@@ -595,13 +670,7 @@ __device__ void sp_ssm_body(const FluidConst& F, const PhasedArgs& a, int r)
             iter++;
             const bool cap = iter > maxIt;
             if (cap || !(Se > Stol)) {
-                if (cap) S.I(IF_META, c) &= ~(int32_t)M_C_SSMSP;
-                S.D(F_::SeSP, c) = Se;
-                S.I(IF_IT2, c) += iter;
-                S.I(IF_IT4, c) += f.it_rr;
-#pragma unroll
-                for (int i = 0; i < NC; i++) S.D(F_::Ks + i, c) = f.Ks[i];
-                store_split(f, S, c);
+                sp_ssm_store(f, S, c, Se, iter, cap);
                 c = a.L.take(list, n);
                 if (c >= 0) load();
             }
@@ -739,8 +808,11 @@ __device__ __forceinline__ void load_split_cell(CellFlash<NC>& f, const PhasedAr
     load_split(f, S, c);
 }
 
-// Start of SplitNR (src/MixtureComp.cpp:2059-2069): n = nu x and the
-// residual; converged cells finish PhaseSplit here, the rest go to Newton.
+// Start of SplitNR (src/MixtureComp.cpp:2059-2069): n = nu x and the size of
+// the residual, for every cell of the split. Writes only these (the Newton
+// kernel, which takes the same list, finishes cells that start converged):
+// 60 x 220 x 85 warm iteration, 3.05 ms with the whole cell loaded, stored
+// back and appended to a list of its own; the whole iteration 25.6 -> 22.7 ms.
 template <int NC>
 __device__ void sp_nrinit_body(const FluidConst& F, const PhasedArgs& a, int r)
 {
@@ -748,28 +820,25 @@ __device__ void sp_nrinit_body(const FluidConst& F, const PhasedArgs& a, int r)
     const StateBuf& S = a.S;
     OCPF_FOR_ITEMS(a, L_SP_0 + r, c)
     {
-        CellFlash<NC> f(F);
-        uint32_t      meta;
-        load_split_cell(f, a, c, meta);
-        f.ssmsp_realTol = sqrt(S.D(F_::SeSP, c));
-        f.nrsp_conflag  = false;
-        double eNR      = 0;
+        const double P = a.in.P[c], nu0 = S.D(F_::nu0, c), nu1 = S.D(F_::nu1, c);
+        double       x0[NC], x1[NC], f0[NC], f1[NC], eNR = 0;
 #pragma unroll
         for (int i = 0; i < NC; i++) {
-            f.n[0][i] = f.nu[0] * f.x[0][i];
-            f.n[1][i] = f.nu[1] * f.x[1][i];
-            const double res = log(f.fug[1][i] / f.fug[0][i]);
+            x0[i] = S.D(F_::x0 + i, c);
+            x1[i] = S.D(F_::x1 + i, c);
+            f0[i] = S.D(F_::phi0 + i, c) * x0[i] * P;
+            f1[i] = S.D(F_::phi1 + i, c) * x1[i] * P;
+        }
+#pragma unroll
+        for (int i = 0; i < NC; i++) {
+            S.D(F_::n0 + i, c) = nu0 * x0[i];
+            S.D(F_::n1 + i, c) = nu1 * x1[i];
+            const double res   = log(f1[i] / f0[i]);
             eNR += res * res;
         }
-        eNR = sqrt(eNR);
-        if (eNR > F.nrsp_tol) {
-            S.D(F_::eNR0, c) = eNR;
-            store_split(f, S, c);
-            store_book(f, S, c, meta);
-            a.L.push(L_SPNR_0 + r, (int32_t)c);
-        } else {
-            sp_after_nr(f, a, c, meta, r, eNR, 0);
-        }
+        S.D(F_::eNR0, c)    = sqrt(eNR);
+        S.D(F_::rtSSMSP, c) = sqrt(S.D(F_::SeSP, c));
+        S.I(IF_META, c) &= ~(int32_t)M_C_NRSP;
     }
 }
 
@@ -778,19 +847,20 @@ __device__ void sp_nrinit_body(const FluidConst& F, const PhasedArgs& a, int r)
 // for every active lane; a lane whose cell ends its Newton loop finishes it
 // (sp_after_nr) and takes the next cell, so lanes stay busy however
 // unequal the cells' step counts are.
+// The list is the split's own, each cell started by sp_nrinit.
 template <int NC>
 __device__ void sp_nr_body(const FluidConst& F, const PhasedArgs& a, int r)
 {
     using F_ = SF<NC>;
     const StateBuf& S    = a.S;
-    const int       list = L_SPNR_0 + r;
+    const int       list = L_SP_0 + r;
     const uint32_t  n    = a.L.len(list);
     CellFlash<NC>   f(F);
     uint32_t        meta = 0;
     double          res[NC];
     double          eNR0 = 0, eNR = 0;
     int             iter = 0;
-    int64_t         c    = a.L.take(list, n);
+    int64_t         c    = a.L.take_again(list, L_SPNR_0 + r, n);
     auto load = [&]() {
         load_split_cell(f, a, c, meta);
         eNR0 = S.D(F_::eNR0, c);
@@ -825,7 +895,7 @@ __device__ void sp_nr_body(const FluidConst& F, const PhasedArgs& a, int r)
             }
             if (done) {
                 sp_after_nr(f, a, c, meta, r, eNR, iter);
-                c = a.L.take(list, n);
+                c = a.L.take_again(list, L_SPNR_0 + r, n);
                 if (c >= 0) load();
             }
         }

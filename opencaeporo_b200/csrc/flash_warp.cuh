@@ -331,29 +331,18 @@ struct WarpSplit {
         share_phases(ph, aj, bj, zj);
     }
 
-    // SplitSSM2 with UpdateXRR, src/MixtureComp.cpp:1847-1903, 2030-2043
-    // (CellFlash::split_ssm2 with the pieces above). Inside the loop lane
+    // SplitSSM2's iterations with UpdateXRR, src/MixtureComp.cpp:1881-1902,
+    // 2030-2043, from f.Ks while Se exceeds Stol, `iter` steps already taken;
+    // f.ssmsp_conflag falls when the cap ends them. Inside the loop lane
     // (j, i) holds component i's K and z and its x_ji and phi_ji; the state
-    // goes to every lane after the last step.
-    __device__ __forceinline__ void split_ssm2_lanes(bool restart)
+    // goes to every lane after the last step. Returns Se.
+    __device__ __forceinline__ double ssm_steps(double Se, double Stol, int maxIt, int& iter)
     {
-        f.ssmsp_conflag = true;
-        double Se       = 1;
-        double Stol     = f.F.ssmsp_tol2;
-        int    maxIt    = f.F.ssmsp_maxit;
-        if (restart) {
-            Stol *= 1e-1;
-            maxIt *= 2;
-        }
-        if (f.Yt < 1.1) {
-            Stol *= 1e-1;
-            maxIt *= 2;
-        }
-        int          iter = 0;
         double       K    = pick(f.Ks), x1 = 0, x0 = 0, ph = 0, aj = 0, bj = 0, zj = 0;
         const double    z = pick(f.zi), P = f.P;
         double          nu0   = f.nu[0];
         int             it_rr = 0;
+        const int       iter0 = iter;
         const bool      zok = __all_sync(WARP_ALL, z == 0 || (z > 0x1p-300 && z < 0x1p100));
         const LaneConst lc  = lane_const();
         while (Se > Stol) {
@@ -371,8 +360,7 @@ struct WarpSplit {
             const double recv = __shfl_xor_sync(WARP_ALL, half ? fg : ph, 16);
             const double quo  = div1(half ? ph : recv, half ? recv : fg);
             const double dq   = quo - 1, dq2 = dq * dq;
-            // the next step's bracket beside this step's residual sum
-            K  = __shfl_sync(WARP_ALL, quo, 16 + (q < NC ? q : 0));
+            K = __shfl_sync(WARP_ALL, quo, 16 + (q < NC ? q : 0));
             double r2[NC];
             read(exchange(dq2), r2);
             Se = 0;
@@ -384,7 +372,7 @@ struct WarpSplit {
                 break;
             }
         }
-        if (iter > 0) {
+        if (iter > iter0) {
             f.nu[0] = nu0;
             f.nu[1] = 1 - nu0;
 #pragma unroll
@@ -395,9 +383,29 @@ struct WarpSplit {
             }
             share_phases(ph, aj, bj, zj);
         }
+        f.it_rr += it_rr;
+        return Se;
+    }
+
+    // SplitSSM2, src/MixtureComp.cpp:1847-1903 (CellFlash::split_ssm2)
+    __device__ __forceinline__ void split_ssm2_lanes(bool restart)
+    {
+        f.ssmsp_conflag = true;
+        double Se       = 1;
+        double Stol     = f.F.ssmsp_tol2;
+        int    maxIt    = f.F.ssmsp_maxit;
+        if (restart) {
+            Stol *= 1e-1;
+            maxIt *= 2;
+        }
+        if (f.Yt < 1.1) {
+            Stol *= 1e-1;
+            maxIt *= 2;
+        }
+        int iter = 0;
+        Se       = ssm_steps(Se, Stol, maxIt, iter);
         f.ssmsp_realTol = sqrt(Se);
         f.it_ssmsp += iter;
-        f.it_rr += it_rr;
     }
 
     // RachfordRice2, src/MixtureComp.cpp:1907-1959 (CellFlash::rachford_rice2):
