@@ -16,8 +16,7 @@
 //
 // Measured on B200, one warp: a dependent division 111 -> 72 cycles (81 with
 // its range test); twelve independent ones 1,344 -> 602 cycles (each `/`
-// brings a branch of its own, so that no two overlap; div_n tests all
-// operands once).
+// brings a branch of its own, so that no two overlap).
 #pragma once
 
 #include <cstdint>
@@ -72,20 +71,6 @@ __device__ __forceinline__ double div1(double a, double b)
     double q = div_core(a, b);
     div_redo(!(div_mid(a) & div_mid(b)) | div_ones(b), a, b, q);
     return q;
-}
-
-// q[i] = a[i] / b[i]
-template <int N>
-__device__ __forceinline__ void div_n(const double (&a)[N], const double (&b)[N], double (&q)[N])
-{
-    bool ok = true;
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-        q[i] = div_core(a[i], b[i]);
-        ok   = ok & div_mid(a[i]) & div_mid(b[i]) & !div_ones(b[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < N; i++) div_redo(!ok, a[i], b[i], q[i]);
 }
 
 }  // namespace ocpf

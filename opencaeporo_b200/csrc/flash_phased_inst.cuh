@@ -20,9 +20,13 @@
 namespace ocpf {
 
 constexpr int kNC = OCPF_NC;
-// The split's iterations partly on whole warps: where the results keep their
-// bits (beyond 6 components the compiler rounds the two forms differently).
-constexpr bool kSplitWarp = kNC <= 6;
+// Calls up to this many cells take the split's iterations partly on whole
+// warps with 9 and 12 components too: the Newton step of 17,081 bulks of 9
+// components 5.7 -> 5.0 ms. In larger calls the trial rounds' whole-warp
+// kernels, at the side streams' priority, hold the SMs while the later trials
+// and round 0 wait: IMPEC of 99,029 bulks 6.4 -> 6.9 ms, so those keep one lane
+// per cell.
+constexpr int64_t kSplitWarpCells = 32768;
 
 #define K128 __global__ void __launch_bounds__(128)
 K128 KP(init)(const __grid_constant__ FluidConst F, const PhasedArgs a) { init_body<kNC>(F, a); }
@@ -87,12 +91,9 @@ void OCPF_CAT(split_round_, OCPF_NC)(const FluidConst& F, const PhasedArgs& a, c
                                     int bp, int gs, int gnr, int gw)
 {
     KP(sp_prep)<<<gp, bp, 0, st>>>(F, a, r);
-    if constexpr (kSplitWarp) {
-        KP(sp_ssm)<<<gs, 128, 0, st>>>(F, a, r, 4u * (uint32_t)gw);
-        KP(sp_ssm_warp)<<<gw, 128, 0, st>>>(F, a, r);
-    } else {
-        KP(sp_ssm)<<<gs, 128, 0, st>>>(F, a, r, 0u);
-    }
+    const uint32_t park = kNC <= 6 || a.count <= kSplitWarpCells ? 4u * (uint32_t)gw : 0u;
+    KP(sp_ssm)<<<gs, 128, 0, st>>>(F, a, r, park);
+    if (park) KP(sp_ssm_warp)<<<gw, 128, 0, st>>>(F, a, r);
     KP(sp_nrinit)<<<gp, bp, 0, st>>>(F, a, r);
     KP(sp_nr)<<<gnr, 128, 0, st>>>(F, a, r);
 }

@@ -560,11 +560,16 @@ __device__ __forceinline__ void sp_ssm_store(const CellFlash<NC>& f, const State
 }
 
 // Split lists of at most SSM_SMALL cells per warp of the whole-warp kernel go
-// to it at once; of longer ones it finishes what a warp of the one-lane kernel
-// is left with when the list is used up and it holds at most SSM_TAIL cells.
-// One lane takes 7 us a step (6 components; its warp's other lanes idle or in
-// other branches), the whole warp 2.6 us.
-constexpr int SSM_SMALL = 2, SSM_TAIL = 3;
+// to it at once. Of lists of up to SSM_SHARE cells per warp it finishes what a
+// warp of the one-lane kernel is left with once the list is used up: when it
+// holds at most SSM_TAIL cells, or SSM_LATE steps later. One lane takes 7 us a
+// step with 6 components, 12 us with 9 (20 in a full warp of cells in different
+// branches); the whole warp 2.6 and 3.1 us, but for one cell. Most splits take
+// 25 steps, a few percent of warm states of 9 components 100 to 201. Measured,
+// 9 components: lists of 7,000 and 10,000 cells 5.7 -> 4.8 ms (the Newton step
+// of 17,081 bulks); a list of 31,000 handed over as well 6.4 -> 6.7 ms
+// (IMPEC, 99,029 bulks), so longer lists stay with the one-lane kernel.
+constexpr int SSM_SMALL = 3, SSM_SHARE = 8, SSM_TAIL = 3, SSM_LATE = 40;
 
 // SplitSSM2's iterations with one warp per cell (flash_warp.cuh), for the
 // cells of list L_SP_r when it is short, else for those the one-lane kernel
@@ -616,8 +621,9 @@ __device__ void sp_ssm_body(const FluidConst& F, const PhasedArgs& a, int r, uin
     const uint32_t  n    = a.L.len(list);
     CellFlash<NC>   f(F);  // holds z, K, x, phi, nu, Aj/Bj/Zj, sA, Bi
     double          Stol = 0;
-    int             maxIt = 0, iter = 0;
+    int             maxIt = 0, iter = 0, late = 0;
     if (n <= SSM_SMALL * park) return;
+    if (n > SSM_SHARE * park) park = 0;
     int64_t         c     = a.L.take(list, n);
     auto load = [&]() {
         f.P = a.in.P[c];
@@ -638,8 +644,8 @@ __device__ void sp_ssm_body(const FluidConst& F, const PhasedArgs& a, int r, uin
     while (true) {
         const uint32_t held = __ballot_sync(0xffffffffu, c >= 0);
         if (held == 0) break;
-        if (park && __popc(held) <= SSM_TAIL) {
-            // lanes without a cell found the list used up
+        late += held != 0xffffffffu;  // a lane without a cell found the list used up
+        if (park && (__popc(held) <= SSM_TAIL || late > SSM_LATE)) {
             if (c >= 0) {
 #pragma unroll
                 for (int i = 0; i < NC; i++) S.D(F_::Ks + i, c) = f.Ks[i];
