@@ -41,6 +41,16 @@ __device__ __forceinline__ double phi_term(double bi, double ti, double ia, doub
 {
     return exp(bi * zm1 - L1 - cf * (2 * ti * ia - bi) * L2);
 }
+// phi_term with every rounding written out (PrCubic::Fixed's reason)
+template <bool FIXED>
+__device__ __forceinline__ double phi_term_of(double bi, double ti, double ia, double zm1, double L1, double cf,
+                                              double L2)
+{
+    if constexpr (FIXED)
+        return exp(__fma_rn(-__dmul_rn(cf, __fma_rn(__dmul_rn(2, ti), ia, -bi)), L2, __fma_rn(bi, zm1, -L1)));
+    else
+        return phi_term(bi, ti, ia, zm1, L1, cf, L2);
+}
 
 // The per-phase pieces of CalFugPhi: q = 0: ln(Z - b), 1: ln((Z + d1 b) /
 // (Z + d2 b)), 2: 1 / b, 3: 1 / a. One division and at most one logarithm
@@ -57,15 +67,15 @@ __device__ __forceinline__ double fug_piece(int q, double zj, double aj, double 
 
 // CalFugPhi (src/MixtureComp.cpp:993-1101): the fugacity coefficients phi
 // and fugacities f = phi x P of composition xj (phiT may be null), with the
-// mixture's a, b and Z (SolEoS).
-template <int NC>
+// mixture's a, b and Z (SolEoS). FIXED: PrCubic::Fixed's roundings.
+template <int NC, bool FIXED = false>
 __device__ __forceinline__ void fug_phi(const FluidConst& F, const double* sA, const double* Bi, double P,
                                         const double* xj, double* phiT, double* fugT, double& aj,
                                         double& bj, double& zj)
 {
     double t[NC];
     mix_ab<NC>(F, sA, Bi, xj, t, aj, bj);
-    zj               = sol_eos(aj, bj);
+    zj               = sol_eos<FIXED>(aj, bj);
     const double L1  = fug_piece(0, zj, aj, bj);
     const double L2  = fug_piece(1, zj, aj, bj);
     const double ib  = fug_piece(2, zj, aj, bj);
@@ -74,7 +84,7 @@ __device__ __forceinline__ void fug_phi(const FluidConst& F, const double* sA, c
     const double zm1 = zj - 1;
 #pragma unroll
     for (int i = 0; i < NC; i++) {
-        const double ph = phi_term(Bi[i] * ib, t[i], ia, zm1, L1, cf, L2);
+        const double ph = phi_term_of<FIXED>(Bi[i] * ib, t[i], ia, zm1, L1, cf, L2);
         if (phiT) phiT[i] = ph;
         if (fugT) fugT[i] = ph * xj[i] * P;
     }

@@ -49,6 +49,30 @@ struct PrCubic {
         Q3 = Q * Q * Q;
         M  = R * R - Q3;
     }
+    // The same with every rounding written out, so that kernels which have to
+    // agree bit for bit (the split's substitution on one lane and on a whole
+    // warp) do not depend on what the compiler fuses: it shares d1 d2 b b
+    // between b and c, rounded, in one kernel, and fuses it into b in another.
+    struct Fixed {};
+    __device__ __forceinline__ PrCubic(double aj, double bj, Fixed)
+    {
+        const double w = __dmul_rn(__dmul_rn(D1TD2, bj), bj), b1 = __dadd_rn(bj, 1);
+        a  = __fma_rn(D1PD2 - 1, bj, -1);
+        b  = __fma_rn(-__dmul_rn(D1PD2, bj), b1, __dadd_rn(aj, w));
+        c  = -__fma_rn(aj, bj, __dmul_rn(w, b1));
+        Q  = div_const(__fma_rn(a, a, -__dmul_rn(3, b)), 9, RCP9);
+        R  = div_const(__fma_rn(27, c, __fma_rn(__dmul_rn(2 * a, a), a, -__dmul_rn(__dmul_rn(9, a), b))), 54, RCP54);
+        Q3 = __dmul_rn(__dmul_rn(Q, Q), Q);
+        M  = __fma_rn(R, R, -Q3);
+    }
+    template <bool FIXED>
+    static __device__ __forceinline__ PrCubic of(double aj, double bj)
+    {
+        if constexpr (FIXED)
+            return PrCubic(aj, bj, Fixed());
+        else
+            return PrCubic(aj, bj);
+    }
     // Root k (0, 1, 2) of the trigonometric form (M <= 0), polished; theta =
     // acos(R / sqrt(Q^3)), with the reference's truncated pi.
     __device__ __forceinline__ double trig_root(int k, double theta) const
@@ -112,9 +136,10 @@ __device__ __forceinline__ double pick_root(double z0, double z1, double z2, dou
 // trigonometric roots with the reference's truncated pi, Newton polish, and
 // for three roots the Gibbs-energy choice between the smallest and largest
 // (SolEoS + CubicRoot, src/MixtureComp.cpp:889-914, 4999-5056).
+template <bool FIXED = false>
 __device__ __forceinline__ double sol_eos(double aj, double bj)
 {
-    const PrCubic cu(aj, bj);
+    const PrCubic cu = PrCubic::of<FIXED>(aj, bj);
     if (cu.M <= 0) {
         const double theta = acos(cu.R / sqrt(cu.Q3));
         const double z0    = cu.trig_root(0, theta);
@@ -131,11 +156,13 @@ __device__ __forceinline__ double sol_eos(double aj, double bj)
 // (returns true), or both the single real root (returns false), on every
 // lane of `mask`. The group has 16 lanes from `base`; its lanes 0, 1 and 2 each polish
 // one of the three trigonometric roots; even and odd lanes form one cube root
-// each of Cardano's form. Same values as sol_eos, bit for bit.
+// each of Cardano's form. Same values as sol_eos: with FIXED bit for bit,
+// otherwise but for what the compiler fuses in the cubic's coefficients.
+template <bool FIXED>
 __device__ __forceinline__ bool root_pair_group(double aj, double bj, unsigned mask, int base, int rank, double& zmin,
                                                 double& zmax)
 {
-    const PrCubic cu(aj, bj);
+    const PrCubic cu = PrCubic::of<FIXED>(aj, bj);
     if (cu.M <= 0) {
         // both square roots at once, on different lanes
         const double rt    = sqrt((rank & 8) ? cu.Q : cu.Q3);

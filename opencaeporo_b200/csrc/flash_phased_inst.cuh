@@ -48,7 +48,7 @@ K128 KP(sta_nr)(const __grid_constant__ FluidConst F, const PhasedArgs a, int k,
 K128 KP(sp_prep)(const __grid_constant__ FluidConst F, const PhasedArgs a, int r) { sp_prep_body<kNC>(F, a, r); }
 K128 KP(sp_ssm)(const __grid_constant__ FluidConst F, const PhasedArgs a, int r, uint32_t park)
 {
-    sp_ssm_body<kNC>(F, a, r, park);
+    sp_ssm_body<kNC, true>(F, a, r, park);
 }
 __global__ void __launch_bounds__(128, 4) KP(sp_ssm_warp)(const __grid_constant__ FluidConst F, const PhasedArgs a, int r)
 {

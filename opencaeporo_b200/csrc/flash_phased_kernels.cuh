@@ -573,7 +573,7 @@ constexpr int SSM_SMALL = 3, SSM_SHARE = 8, SSM_TAIL = 3, SSM_LATE = 40;
 
 // SplitSSM2's iterations with one warp per cell (flash_warp.cuh), for the
 // cells of list L_SP_r when it is short, else for those the one-lane kernel
-// left on L_SPNR_r. `warps`: this kernel's whole grid.
+// left on L_SPNR_r.
 template <int NC>
 __device__ __noinline__ void sp_ssm_on_warp(const FluidConst& F, const PhasedArgs& a, int64_t c)
 {
@@ -593,7 +593,7 @@ __device__ __noinline__ void sp_ssm_on_warp(const FluidConst& F, const PhasedArg
     f.nu[0]         = 0;
     WarpSplit<NC> w(f);
     int           iter = 0;
-    const double  Se   = w.ssm_steps(HUGE_VAL, S.D(F_::Stol, c), S.I(IF_MAXIT, c), iter);
+    const double  Se   = w.template ssm_steps<true>(HUGE_VAL, S.D(F_::Stol, c), S.I(IF_MAXIT, c), iter);
     if ((threadIdx.x & 31) == 0) sp_ssm_store(f, S, c, Se, iter, !f.ssmsp_conflag);
     __syncwarp();
 }
@@ -611,8 +611,11 @@ __device__ void sp_ssm_warp_body(const FluidConst& F, const PhasedArgs& a, int r
 // SplitSSM2's iterations (src/MixtureComp.cpp:1881-1902) on a persistent
 // grid: per turn, Rachford-Rice, the phase compositions, the fugacities of
 // both phases, and the K update. With `park` (the warps of the whole-warp
-// kernel that follows; 0: none) short lists and tails are left to it.
-template <int NC>
+// kernel that follows; 0: none) short lists and tails are left to it. Which
+// cells these are depends on the list's length and on the order of the appends,
+// so both kernels form the steps with the same roundings (FIXED) and a cell's
+// bits do not depend on its route.
+template <int NC, bool FIXED = false>
 __device__ void sp_ssm_body(const FluidConst& F, const PhasedArgs& a, int r, uint32_t park = 0)
 {
     using F_ = SF<NC>;
@@ -665,8 +668,8 @@ __device__ void sp_ssm_body(const FluidConst& F, const PhasedArgs& a, int r, uin
                 f.x[0][i]        = f.Ks[i] * f.x[1][i];
             }
             double fug0[NC], fug1[NC];
-            fug_phi<NC>(F, f.sA, f.Bi, f.P, f.x[0], f.phi[0], fug0, f.Aj[0], f.Bj[0], f.Zj[0]);
-            fug_phi<NC>(F, f.sA, f.Bi, f.P, f.x[1], f.phi[1], fug1, f.Aj[1], f.Bj[1], f.Zj[1]);
+            fug_phi<NC, FIXED>(F, f.sA, f.Bi, f.P, f.x[0], f.phi[0], fug0, f.Aj[0], f.Bj[0], f.Zj[0]);
+            fug_phi<NC, FIXED>(F, f.sA, f.Bi, f.P, f.x[1], f.phi[1], fug1, f.Aj[1], f.Bj[1], f.Zj[1]);
             double Se = 0;
 #pragma unroll
             for (int i = 0; i < NC; i++) {

@@ -220,6 +220,7 @@ struct WarpSplit {
     // division and one logarithm per lane form, side by side, CalFugPhi's
     // pieces for the smallest root (lanes 0-3), for the largest (4-7) and
     // the pieces of the choice between the two (8-10).
+    template <bool FIXED>
     __device__ __forceinline__ double fug_lane(const double (&xj)[NC], const LaneConst& lc, double& aj, double& bj,
                                                double& zj) const
     {
@@ -238,7 +239,7 @@ struct WarpSplit {
         }
         const int  base = half << 4;
         double     zmin, zmax;
-        const bool three = root_pair_group(aj, bj, hmask, base, q, zmin, zmax);
+        const bool three = root_pair_group<FIXED>(aj, bj, hmask, base, q, zmin, zmax);
         __syncwarp();
         // num = (n1 b + u1) (n2 b + u2), den = (d1 b + w1) (d2 b + w2) with
         // the coefficients of the lane's piece (LaneConst); a factor that a
@@ -270,7 +271,7 @@ struct WarpSplit {
         const double ia  = __shfl_sync(WARP_ALL, piece, base + 3);
         const double cf  = div_const(aj, D1MD2, RCPD1MD2) * ib;
         const double zm1 = zj - 1;
-        return phi_term(lc.Bi * ib, tq, ia, zm1, L1, cf, L2);
+        return phi_term_of<FIXED>(lc.Bi * ib, tq, ia, zm1, L1, cf, L2);
     }
 
     // One phase of CalFugPhi (src/MixtureComp.cpp:993-1101) on each half:
@@ -335,7 +336,9 @@ struct WarpSplit {
     // 2030-2043, from f.Ks while Se exceeds Stol, `iter` steps already taken;
     // f.ssmsp_conflag falls when the cap ends them. Inside the loop lane
     // (j, i) holds component i's K and z and its x_ji and phi_ji; the state
-    // goes to every lane after the last step. Returns Se.
+    // goes to every lane after the last step. Returns Se. FIXED:
+    // PrCubic::Fixed's roundings, the one-lane kernel's (sp_ssm_body).
+    template <bool FIXED>
     __device__ __forceinline__ double ssm_steps(double Se, double Stol, int maxIt, int& iter)
     {
         double       K    = pick(f.Ks), x1 = 0, x0 = 0, ph = 0, aj = 0, bj = 0, zj = 0;
@@ -353,7 +356,7 @@ struct WarpSplit {
             x0 = K * x1;
             double xj[NC];
             gather(half ? x1 : x0, xj);
-            ph = fug_lane(xj, lc, aj, bj, zj);
+            ph = fug_lane<FIXED>(xj, lc, aj, bj, zj);
             // lane i: component i's squared fugacity-ratio residual; lane
             // 16 + i: its new K (one division on every lane)
             const double fg   = ph * (half ? x1 : x0) * P;
@@ -403,7 +406,7 @@ struct WarpSplit {
             maxIt *= 2;
         }
         int iter = 0;
-        Se       = ssm_steps(Se, Stol, maxIt, iter);
+        Se       = ssm_steps<false>(Se, Stol, maxIt, iter);
         f.ssmsp_realTol = sqrt(Se);
         f.it_ssmsp += iter;
     }
