@@ -13,7 +13,7 @@
 //   strict round k (StableSSM trial k + StableNR), k = 0..3:
 //                 prep -> persistent SSM -> verdict -> Newton
 //   split         (SplitSSM2 + SplitNR, first try):
-//                 prep -> persistent SSM -> SSM of short lists and tails, one
+//                 prep -> persistent SSM, short lists and long cells on one
 //                 warp per cell -> Newton start -> persistent Newton
 //   restarts      cells whose split restarts: the rest of PhaseSplit, one
 //                 warp per cell (flash_warp.cuh)
@@ -88,7 +88,7 @@ enum ListId : int {
     L_STA_0, L_STA_1, L_STA_2, L_STA_3,
     L_NRSTA_0, L_NRSTA_1, L_NRSTA_2, L_NRSTA_3,
     L_SP_0, L_SP_LEARN, L_SP_T0, L_SP_T1, L_SP_T2, L_SP_T3,
-    // the split's tails for the whole-warp kernel; the consumer head counts
+    // the cells handed to the split's whole-warp kernel; the consumer head counts
     // the Newton kernel's second pass over the split's own list
     L_SPNR_0, L_SPNR_LEARN, L_SPNR_T0, L_SPNR_T1, L_SPNR_T2, L_SPNR_T3,
     L_SLOW, L_SLOW_T0, L_SLOW_T1, L_SLOW_T2, L_SLOW_T3,

@@ -20,14 +20,6 @@
 namespace ocpf {
 
 constexpr int kNC = OCPF_NC;
-// Calls up to this many cells take the split's iterations partly on whole
-// warps with 9 and 12 components too: the Newton step of 17,081 bulks of 9
-// components 5.7 -> 5.0 ms. In larger calls the trial rounds' whole-warp
-// kernels, at the side streams' priority, hold the SMs while the later trials
-// and round 0 wait: IMPEC of 99,029 bulks 6.4 -> 6.9 ms, so those keep one lane
-// per cell.
-constexpr int64_t kSplitWarpCells = 32768;
-
 #define K128 __global__ void __launch_bounds__(128)
 K128 KP(init)(const __grid_constant__ FluidConst F, const PhasedArgs a) { init_body<kNC>(F, a); }
 K128 KP(s01_prep)(const __grid_constant__ FluidConst F, const PhasedArgs a, int k) { s01_prep_body<kNC>(F, a, k); }
@@ -46,13 +38,15 @@ K128 KP(sta_nr)(const __grid_constant__ FluidConst F, const PhasedArgs a, int k,
     sta_nr_body<kNC>(F, a, k, list, fallback);
 }
 K128 KP(sp_prep)(const __grid_constant__ FluidConst F, const PhasedArgs a, int r) { sp_prep_body<kNC>(F, a, r); }
-K128 KP(sp_ssm)(const __grid_constant__ FluidConst F, const PhasedArgs a, int r, uint32_t park)
+K128 KP(sp_ssm)(const __grid_constant__ FluidConst F, const PhasedArgs a, int r, uint32_t direct,
+                uint32_t most)
 {
-    sp_ssm_body<kNC, true>(F, a, r, park);
+    sp_ssm_body<kNC, true>(F, a, r, direct, most);
 }
-__global__ void __launch_bounds__(128, 4) KP(sp_ssm_warp)(const __grid_constant__ FluidConst F, const PhasedArgs a, int r)
+__global__ void __launch_bounds__(128, 4) KP(sp_ssm_warp)(const __grid_constant__ FluidConst F, const PhasedArgs a, int r,
+                                                       uint32_t direct)
 {
-    sp_ssm_warp_body<kNC>(F, a, r);
+    sp_ssm_warp_body<kNC>(F, a, r, direct);
 }
 K128 KP(sp_nrinit)(const __grid_constant__ FluidConst F, const PhasedArgs a, int r) { sp_nrinit_body<kNC>(F, a, r); }
 K128 KP(sp_nr)(const __grid_constant__ FluidConst F, const PhasedArgs a, int r) { sp_nr_body<kNC>(F, a, r); }
@@ -86,14 +80,47 @@ int OCPF_CAT(persistent_grid_, OCPF_NC)(const void* k, int sms, int pct)
     return sms * use;
 }
 
-// One split round: set-up, successive substitution, Newton.
+// Where the split's substitution runs, by the cells of the call in units of
+// the whole-warp kernel's 16 warps an SM (w = 2,368 on 148 SMs; a list has at
+// most the call's cells): up to kWarpAll w on that kernel alone; up to
+// kWarpHand w lists of up to 3 cells a warp go to it at once, and of lists of
+// up to 32 a warp the cells that take more than SSM_STEPS; larger calls stay
+// on one lane per cell. One lane per cell -> so, warm flash:
+//   3 components: 924 bulks 0.28 -> 0.24 ms, but a list of 3 w 0.30 -> 0.37,
+//     and launched behind the one-lane kernel it costs calls of 8,000 to
+//     100,000 bulks 2 to 13 % (blocks of 128 registers a thread that find
+//     nothing to do; a small kernel in its place costs nothing).
+//   6: 924 and 2,880 bulks 0.98 -> 0.82 and 1.13 -> 1.06 ms, a list of 3.2 w
+//     1.26 -> 1.35. Handed over: fresh fast flash of 12,000 and 40,000 cells
+//     12.8 -> 10.5 and 16.1 -> 15.0, warm ones of 8,000 to 60,000 bulks within
+//     2 % (with four blocks an SM 14.5 and 5 % slower).
+//   9: 924, 2,880, 7,700 and 16,632 bulks 3.7 -> 2.5, 4.3 -> 3.1, 4.7 -> 3.6
+//     and 5.3 -> 4.5 ms. Handed over: 24,960, 39,960 and 54,243 bulks 5.5 ->
+//     4.7, 5.9 -> 5.2 and 6.0 -> 5.7, 99,200 6.7 -> 7.1.
+//   12: 924, 7,700 and 16,632 bulks 18.2 -> 13.3, 19.7 -> 16.9 and 20.8 ->
+//     18.7 ms. Handed over: 24,960 and 54,243 bulks 22.5 -> 19.9 and 25.1 ->
+//     23.7, 99,200 the same.
+constexpr int kWarpAll  = kNC <= 3 ? 1 : (kNC <= 6 ? 2 : 7);
+constexpr int kWarpHand = kNC <= 3 ? 0 : (kNC <= 6 ? 1 << 20 : 24);  // 6: every size
+
+// One split round: set-up, successive substitution, Newton. sms: the SMs.
 void OCPF_CAT(split_round_, OCPF_NC)(const FluidConst& F, const PhasedArgs& a, cudaStream_t st, int r, int gp,
-                                    int bp, int gs, int gnr, int gw)
+                                    int bp, int gs, int gnr, int sms)
 {
     KP(sp_prep)<<<gp, bp, 0, st>>>(F, a, r);
-    const uint32_t park = kNC <= 6 || a.count <= kSplitWarpCells ? 4u * (uint32_t)gw : 0u;
-    KP(sp_ssm)<<<gs, 128, 0, st>>>(F, a, r, park);
-    if (park) KP(sp_ssm_warp)<<<gw, 128, 0, st>>>(F, a, r);
+    const int64_t w = 16 * (int64_t)sms;
+    if (a.count <= kWarpAll * w) {
+        KP(sp_ssm_warp)<<<(unsigned)std::min<int64_t>(4 * sms, (a.count + 3) / 4), 128, 0, st>>>(F, a, r, ~0u);
+    } else if (a.count <= kWarpHand * w) {
+        // blocks an SM: one in a trial's round, which runs beside the main
+        // sequence and would hold its SMs, else two or four
+        const int      blocks = r >= TRIAL_ROUND0 ? sms : (kNC <= 6 ? 2 * sms : 4 * sms);
+        const uint32_t direct = 3u * 4u * (uint32_t)blocks, most = 32u * 4u * (uint32_t)blocks;
+        KP(sp_ssm)<<<gs, 128, 0, st>>>(F, a, r, direct, most);
+        KP(sp_ssm_warp)<<<blocks, 128, 0, st>>>(F, a, r, direct);
+    } else {
+        KP(sp_ssm)<<<gs, 128, 0, st>>>(F, a, r, 0u, 0u);
+    }
     KP(sp_nrinit)<<<gp, bp, 0, st>>>(F, a, r);
     KP(sp_nr)<<<gnr, 128, 0, st>>>(F, a, r);
 }
@@ -142,7 +169,7 @@ cudaError_t OCPF_CAT(launch_phased_nc, OCPF_NC)(const FluidConst& F, const Phase
         // (with PH_DEFER their split waits until trial 1 has run, below)
         const int gl = (int)std::min<int64_t>((a.count + LEARN_TILE - 1) / LEARN_TILE, (int64_t)sms * 4);
         KP(learn)<<<gl, 128, sizeof(LearnSmem), st>>>(F, a);
-        if (!defer) OCPF_CAT(split_round_, OCPF_NC)(F, a, st, LEARN_ROUND, gp, bp, g_sp, g_spnr, sms * 4);
+        if (!defer) OCPF_CAT(split_round_, OCPF_NC)(F, a, st, LEARN_ROUND, gp, bp, g_sp, g_spnr, sms);
     }
     for (int k = 0; k < 2; k++) {
         KP(s01_prep)<<<gp, bp, 0, st>>>(F, a, k);
@@ -181,7 +208,7 @@ cudaError_t OCPF_CAT(launch_phased_nc, OCPF_NC)(const FluidConst& F, const Phase
                 cudaEventRecord(side->fork[k], st);
                 cudaStreamWaitEvent(ss, side->fork[k], 0);
             }
-            OCPF_CAT(split_round_, OCPF_NC)(F, a, ss, TRIAL_ROUND0 + k, gp, bp, g_sp, g_spnr, sms * 4);
+            OCPF_CAT(split_round_, OCPF_NC)(F, a, ss, TRIAL_ROUND0 + k, gp, bp, g_sp, g_spnr, sms);
             if (t.slow_threads)
                 KP(slow_thread)<<<gp, bp, 0, ss>>>(F, a, L_SLOW_T0 + k);
             else
@@ -200,7 +227,7 @@ cudaError_t OCPF_CAT(launch_phased_nc, OCPF_NC)(const FluidConst& F, const Phase
                 cudaEventRecord(side->fork[0], st);
                 cudaStreamWaitEvent(ss, side->fork[0], 0);
             }
-            OCPF_CAT(split_round_, OCPF_NC)(F, a, ss, LEARN_ROUND, gp, bp, g_sp, g_spnr, sms * 4);
+            OCPF_CAT(split_round_, OCPF_NC)(F, a, ss, LEARN_ROUND, gp, bp, g_sp, g_spnr, sms);
             PhasedArgs b = a;
             b.sdup       = 1;
             b.opts &= ~(PH_EARLY | PH_DEFER);
@@ -209,7 +236,7 @@ cudaError_t OCPF_CAT(launch_phased_nc, OCPF_NC)(const FluidConst& F, const Phase
         }
     }
     if (defer && side) cudaStreamWaitEvent(st, side->join[0], 0);
-    for (int r = 0; r < SPLIT_ROUNDS; r++) OCPF_CAT(split_round_, OCPF_NC)(F, a, st, r, gp, bp, g_sp, g_spnr, sms * 4);
+    for (int r = 0; r < SPLIT_ROUNDS; r++) OCPF_CAT(split_round_, OCPF_NC)(F, a, st, r, gp, bp, g_sp, g_spnr, sms);
     if (marks) cudaEventRecord(marks[0], st);
     if (t.slow_threads)
         KP(slow_thread)<<<gp, bp, 0, st>>>(F, a, L_SLOW);

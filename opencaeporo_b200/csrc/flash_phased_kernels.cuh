@@ -559,21 +559,16 @@ __device__ __forceinline__ void sp_ssm_store(const CellFlash<NC>& f, const State
     store_split(f, S, c);
 }
 
-// Split lists of at most SSM_SMALL cells per warp of the whole-warp kernel go
-// to it at once. Of lists of up to SSM_SHARE cells per warp it finishes what a
-// warp of the one-lane kernel is left with once the list is used up: when it
-// holds at most SSM_TAIL cells, or SSM_LATE steps later. One lane takes 7 us a
-// step with 6 components, 12 us with 9 (20 in a full warp of cells in different
-// branches); the whole warp 2.6 and 3.1 us, but for one cell. Most splits take
-// 25 steps, a few percent of warm states of 9 components 100 to 201. Measured,
-// 9 components: lists of 7,000 and 10,000 cells 5.7 -> 4.8 ms (the Newton step
-// of 17,081 bulks); a list of 31,000 handed over as well 6.4 -> 6.7 ms
-// (IMPEC, 99,029 bulks), so longer lists stay with the one-lane kernel.
-constexpr int SSM_SMALL = 3, SSM_SHARE = 8, SSM_TAIL = 3, SSM_LATE = 40;
+// A cell that the one-lane kernel has iterated this often goes on in the
+// whole-warp kernel, where there is one (split_round_). Most splits take 25
+// steps, a few percent of warm states of 9 components 100 to 201, and a lane
+// takes 7 us a step with 6 components and 12 us with 9 (20 in a full warp of
+// cells in different branches), the whole warp 2.6 and 3.1 us.
+constexpr int SSM_STEPS = 40;
 
 // SplitSSM2's iterations with one warp per cell (flash_warp.cuh), for the
-// cells of list L_SP_r when it is short, else for those the one-lane kernel
-// left on L_SPNR_r.
+// cells of list L_SP_r when it has at most `direct`, else for those the
+// one-lane kernel handed over on L_SPNR_r.
 template <int NC>
 __device__ __noinline__ void sp_ssm_on_warp(const FluidConst& F, const PhasedArgs& a, int64_t c)
 {
@@ -598,11 +593,10 @@ __device__ __noinline__ void sp_ssm_on_warp(const FluidConst& F, const PhasedArg
     __syncwarp();
 }
 template <int NC>
-__device__ void sp_ssm_warp_body(const FluidConst& F, const PhasedArgs& a, int r)
+__device__ void sp_ssm_warp_body(const FluidConst& F, const PhasedArgs& a, int r, uint32_t direct)
 {
     const uint32_t nw   = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t all  = a.L.len(L_SP_0 + r);
-    const int      list = all <= SSM_SMALL * nw ? L_SP_0 + r : L_SPNR_0 + r;
+    const int      list = a.L.len(L_SP_0 + r) <= direct ? L_SP_0 + r : L_SPNR_0 + r;
     const uint32_t n    = a.L.len(list);
     for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < n; k += nw)
         sp_ssm_on_warp<NC>(F, a, a.L.item(list, k));
@@ -610,13 +604,14 @@ __device__ void sp_ssm_warp_body(const FluidConst& F, const PhasedArgs& a, int r
 
 // SplitSSM2's iterations (src/MixtureComp.cpp:1881-1902) on a persistent
 // grid: per turn, Rachford-Rice, the phase compositions, the fugacities of
-// both phases, and the K update. With `park` (the warps of the whole-warp
-// kernel that follows; 0: none) short lists and tails are left to it. Which
-// cells these are depends on the list's length and on the order of the appends,
-// so both kernels form the steps with the same roundings (FIXED) and a cell's
-// bits do not depend on its route.
+// both phases, and the K update. Lists of at most `direct` cells are left to
+// the whole-warp kernel that follows, and of lists of at most `most` cells the
+// ones that take more than SSM_STEPS (0 and 0: all stay here). The route
+// depends on the list's length, so both kernels form the steps with the same
+// roundings (FIXED), and a cell's bits do not depend on it.
 template <int NC, bool FIXED = false>
-__device__ void sp_ssm_body(const FluidConst& F, const PhasedArgs& a, int r, uint32_t park = 0)
+__device__ void sp_ssm_body(const FluidConst& F, const PhasedArgs& a, int r, uint32_t direct = 0,
+                            uint32_t most = 0)
 {
     using F_ = SF<NC>;
     const StateBuf& S    = a.S;
@@ -624,10 +619,10 @@ __device__ void sp_ssm_body(const FluidConst& F, const PhasedArgs& a, int r, uin
     const uint32_t  n    = a.L.len(list);
     CellFlash<NC>   f(F);  // holds z, K, x, phi, nu, Aj/Bj/Zj, sA, Bi
     double          Stol = 0;
-    int             maxIt = 0, iter = 0, late = 0;
-    if (n <= SSM_SMALL * park) return;
-    if (n > SSM_SHARE * park) park = 0;
-    int64_t         c     = a.L.take(list, n);
+    int             maxIt = 0, iter = 0;
+    if (n <= direct) return;
+    const int hand = n <= most ? SSM_STEPS : 0;
+    int64_t   c    = a.L.take(list, n);
     auto load = [&]() {
         f.P = a.in.P[c];
         load_z<NC>(a, c, f.zi);
@@ -644,21 +639,7 @@ __device__ void sp_ssm_body(const FluidConst& F, const PhasedArgs& a, int r, uin
         f.NP     = 2;
     };
     if (c >= 0) load();
-    while (true) {
-        const uint32_t held = __ballot_sync(0xffffffffu, c >= 0);
-        if (held == 0) break;
-        late += held != 0xffffffffu;  // a lane without a cell found the list used up
-        if (park && (__popc(held) <= SSM_TAIL || late > SSM_LATE)) {
-            if (c >= 0) {
-#pragma unroll
-                for (int i = 0; i < NC; i++) S.D(F_::Ks + i, c) = f.Ks[i];
-                S.I(IF_IT2, c) += iter;
-                S.I(IF_IT4, c) += f.it_rr;
-                S.I(IF_MAXIT, c) = maxIt - iter;
-                a.L.push(L_SPNR_0 + r, (int32_t)c);
-            }
-            break;
-        }
+    while (__any_sync(0xffffffffu, c >= 0)) {
         if (c >= 0) {
             f.rachford_rice2();
 #pragma unroll
@@ -680,6 +661,15 @@ __device__ void sp_ssm_body(const FluidConst& F, const PhasedArgs& a, int r, uin
             const bool cap = iter > maxIt;
             if (cap || !(Se > Stol)) {
                 sp_ssm_store(f, S, c, Se, iter, cap);
+                c = a.L.take(list, n);
+                if (c >= 0) load();
+            } else if (iter == hand) {
+#pragma unroll
+                for (int i = 0; i < NC; i++) S.D(F_::Ks + i, c) = f.Ks[i];
+                S.I(IF_IT2, c) += iter;
+                S.I(IF_IT4, c) += f.it_rr;
+                S.I(IF_MAXIT, c) = maxIt - iter;
+                a.L.push(L_SPNR_0 + r, (int32_t)c);
                 c = a.L.take(list, n);
                 if (c >= 0) load();
             }
