@@ -509,6 +509,14 @@ int ocpf_set_initializer(ocpf_ctx* ctx, const float* params, const float* in_mea
  * reference counterpart (measurement utility). */
 int ocpf_measure_fp64_latency(int device, double* cycles);
 
+/* Evaluates one of the kernels' own divisions on device arrays a, b, q of n
+ * values, so that it can be compared with `/`: form 0 a / b, 1 the guarded and
+ * 2 the unguarded division of the restart path, 3, 4, 5, 6 the division of a by
+ * the constants 3, 9, 54 and d1 - d2 of the cubic and the fugacities, 7 the
+ * error 1 - b y0 of the reciprocal the restart path's division starts from. No
+ * reference counterpart (check). */
+int ocpf_check_division(int form, int64_t n, const double* a, const double* b, double* q, void* stream);
+
 /* ---------------------------------------------------------------------
  * Relative permeability and capillary pressure after the flash
  * (IsoT_FIM::CalKrPc / IsoT_IMPEC::CalKrPc, src/OCPFluidMethod.cpp:

@@ -34,7 +34,7 @@ EXPORTS = ("ocpf_version", "ocpf_status_string", "ocpf_create", "ocpf_destroy",
            "ocpf_flash_fim", "ocpf_flash_fim_host", "ocpf_last_kernel_ms",
            "ocpf_measure_fma_peak", "ocpf_reserve", "ocpf_flash_fim_noalloc",
            "ocpf_mlp_param_count", "ocpf_mlp_forward", "ocpf_mlp_grad", "ocpf_mlp_adam",
-           "ocpf_set_initializer", "ocpf_flash_fim_regions", "ocpf_measure_fp64_latency",
+           "ocpf_set_initializer", "ocpf_flash_fim_regions", "ocpf_measure_fp64_latency", "ocpf_check_division",
            "ocpf_flash_impec", "ocpf_init_flash_fim", "ocpf_init_flash_impec",
            "ocpf_flash_fimn", "ocpf_init_flash_fimn", "ocpf_flash_fim_subset", "ocpf_flash_impec_subset",
            "ocpf_krpc_create", "ocpf_krpc_destroy", "ocpf_cal_krpc", "ocpf_last_launch_count",
@@ -236,6 +236,8 @@ def lib():
     L.ocpf_autotune.restype = C.c_int
     L.ocpf_measure_fp64_latency.argtypes = [C.c_int, C.POINTER(C.c_double)]
     L.ocpf_measure_fp64_latency.restype = C.c_int
+    L.ocpf_check_division.argtypes = [C.c_int, C.c_int64] + [C.c_void_p] * 4
+    L.ocpf_check_division.restype = C.c_int
     L.ocpf_flash_impec.argtypes = [_vp, C.c_int64, C.POINTER(ImpecIn), C.POINTER(Skip), C.POINTER(ImpecOut),
                                    C.c_int, _vp]
     L.ocpf_flash_impec.restype = C.c_int
