@@ -83,17 +83,21 @@ int OCPF_CAT(persistent_grid_, OCPF_NC)(const void* k, int sms, int pct)
 // Where the split's substitution runs, by the cells of the call in units of
 // the whole-warp kernel's 16 warps an SM (w = 2,368 on 148 SMs; a list has at
 // most the call's cells): up to kWarpAll w on that kernel alone; up to
-// kWarpHand w lists of up to 3 cells a warp go to it at once, and of lists of
-// up to 32 a warp the cells that take more than SSM_STEPS; larger calls stay
-// on one lane per cell. One lane per cell -> so, warm flash:
+// kWarpHand w lists of up to 3 cells a warp (with 6 components of two blocks
+// an SM) go to it at once, and of lists of up to 32 a warp the cells that take
+// more than SSM_STEPS; larger calls stay on one lane per cell. One lane per
+// cell -> so, warm flash:
 //   3 components: 924 bulks 0.28 -> 0.24 ms, but a list of 3 w 0.30 -> 0.37,
 //     and launched behind the one-lane kernel it costs calls of 8,000 to
 //     100,000 bulks 2 to 13 % (blocks of 128 registers a thread that find
 //     nothing to do; a small kernel in its place costs nothing).
 //   6: 924 and 2,880 bulks 0.98 -> 0.82 and 1.13 -> 1.06 ms, a list of 3.2 w
-//     1.26 -> 1.35. Handed over: fresh fast flash of 12,000 and 40,000 cells
-//     12.8 -> 10.5 and 16.1 -> 15.0, warm ones of 8,000 to 60,000 bulks within
-//     2 % (with four blocks an SM 14.5 and 5 % slower).
+//     1.26 -> 1.35. Handed over: fresh fast flash of 12,000 and 47,673 cells
+//     13.1 -> 10.5 and 16.6 -> 14.6, warm ones of 8,000 to 60,000 bulks within
+//     2 %. Above kWarpWide w the kernel takes four blocks an SM instead of two:
+//     fresh flash of 47,673 and 90,000 cells 13.5 -> 12.6 and 16.2 -> 15.4, a
+//     warm one of 32,000 bulks the same; one of 17,160 1.39 -> 1.45, and a
+//     fresh one of 11,875 10.5 -> 10.2.
 //   9: 924, 2,880, 7,700 and 16,632 bulks 3.7 -> 2.5, 4.3 -> 3.1, 4.7 -> 3.6
 //     and 5.3 -> 4.5 ms. Handed over: 24,960, 39,960 and 54,243 bulks 5.5 ->
 //     4.7, 5.9 -> 5.2 and 6.0 -> 5.7, 99,200 6.7 -> 7.1.
@@ -102,6 +106,7 @@ int OCPF_CAT(persistent_grid_, OCPF_NC)(const void* k, int sms, int pct)
 //     23.7, 99,200 the same.
 constexpr int kWarpAll  = kNC <= 3 ? 1 : (kNC <= 6 ? 2 : 7);
 constexpr int kWarpHand = kNC <= 3 ? 0 : (kNC <= 6 ? 1 << 20 : 24);  // 6: every size
+constexpr int kWarpWide = kNC <= 6 ? 12 : 0;
 
 // One split round: set-up, successive substitution, Newton. sms: the SMs.
 void OCPF_CAT(split_round_, OCPF_NC)(const FluidConst& F, const PhasedArgs& a, cudaStream_t st, int r, int gp,
@@ -114,10 +119,11 @@ void OCPF_CAT(split_round_, OCPF_NC)(const FluidConst& F, const PhasedArgs& a, c
     } else if (a.count <= kWarpHand * w) {
         // blocks an SM: one in a trial's round, which runs beside the main
         // sequence and would hold its SMs, else two or four
-        const int      blocks = r >= TRIAL_ROUND0 ? sms : (kNC <= 6 ? 2 * sms : 4 * sms);
-        const uint32_t direct = 3u * 4u * (uint32_t)blocks, most = 32u * 4u * (uint32_t)blocks;
-        KP(sp_ssm)<<<gs, 128, 0, st>>>(F, a, r, direct, most);
-        KP(sp_ssm_warp)<<<blocks, 128, 0, st>>>(F, a, r, direct);
+        const bool     trial  = r >= TRIAL_ROUND0;
+        const int      blocks = trial ? sms : (a.count <= kWarpWide * w ? 2 * sms : 4 * sms);
+        const uint32_t warps  = 4u * (uint32_t)(trial || kNC > 6 ? blocks : 2 * sms);  // the limits' unit
+        KP(sp_ssm)<<<gs, 128, 0, st>>>(F, a, r, 3u * warps, 32u * warps);
+        KP(sp_ssm_warp)<<<blocks, 128, 0, st>>>(F, a, r, 3u * warps);
     } else {
         KP(sp_ssm)<<<gs, 128, 0, st>>>(F, a, r, 0u, 0u);
     }

@@ -54,7 +54,7 @@ def test_bits_do_not_depend_on_the_list(nc):
     want = _warm(m, inp, 25 * w)
     # cells that go on past the hand-over are among them
     assert nc == 3 or (want["iters"][2] > 40).sum() > 16
-    runs = [(k * w + d, 100) for k in (1, 2, 3, 7, 8, 16, 24) for d in (0, 1)] + [(40, 100), (5 * w, 50), (9 * w, 50)]
+    runs = [(k * w + d, 100) for k in (1, 2, 3, 7, 8, 12, 16, 24) for d in (0, 1)] + [(40, 100), (5 * w, 50), (9 * w, 50)]
     for n, pct in runs + [(9 * w, 100), (9 * w, 100), (25 * w, 50)]:
         got = _warm(m, inp, n, pct)
         for k, v in got.items():
