@@ -93,10 +93,10 @@ __global__ void __launch_bounds__(256) k_upwind(const ConnDev C, const ocpf_jac_
 // whole call: 11.1 ms with the rows and columns through shared memory (one
 // thread per row, then per column), 9.8 ms with this split reading dSec_dPri
 // directly, 7.2 ms staged, 6.2 ms with the next composition's partials
-// prefetched and the quotients batched (div_by). 100,000 bulks: 3 components
-// at 561,000 bulks 3.47 -> 1.28 ms, 9 components 2.42 -> 1.46 ms, 12
-// components 6.76 -> 3.55 ms. Rows a thread: 4 for 3, 6 and 12 components, 5
-// for 9, where 3 or 4 rows took 2.43 ms.
+// prefetched and the quotients batched (div_by). 3 components, 561,000 bulks:
+// 3.47 -> 1.28 ms; 9 and 12 components, 100,000 bulks: 2.42 -> 1.46 and 6.76 ->
+// 3.55 ms. Rows a thread: 4 for 3, 6 and 12 components, 5 for 9, where 3 or 4
+// rows took 2.43 ms.
 template <int NCOM>
 struct ConnTile {
     static constexpr int NCOL  = NCOM + 1;
@@ -111,7 +111,6 @@ struct ConnTile {
     static constexpr bool   STAGED  = NCOM <= 7;
     static constexpr int    NENT    = NSEC * NCOL;
     static constexpr size_t SEC     = STAGED ? (size_t)2 * NENT * 32 : 0;  // doubles per tile
-    static constexpr size_t XIJ     = (size_t)J_NP * NCOM * 32;
 };
 
 // Per connection and phase, formed once per tile (stage_phase).
